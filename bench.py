@@ -40,7 +40,7 @@ FALLBACK_HBM_GBS = 6650.0
 TOL = 1e-10
 GOLDEN = ROOT / "tests" / "golden"
 # ncu DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of one ILU0
-# application at 64^3 with 8x8 FP64 blocks (its two streamed sweeps), from the
+# application at 64^3 with 8x8 FP64 blocks (its two sweeps), from the
 # committed capture summarised in profiles/sweep_stream_ilu0_64cube_bs8.md
 ILU_APPLY_TRAFFIC_64 = 1_013_952_512  # 439.6 MB forward + 574.3 MB backward
 
@@ -864,7 +864,7 @@ def run_complex(args):
 
 
 def run_apply(args):
-    """The ILU0 application alone (forward + backward streamed sweeps) on the
+    """The ILU0 application alone (forward + backward sweeps) on the
     64^3 8x8 system, `steps` times after `warmup`: the kernel the solve's
     roofline is quoted on, in a short program that profilers can capture."""
     import torch
@@ -894,7 +894,7 @@ def run_apply(args):
     peak, kind = read_peaks()
     nbytes = ilu_apply_bytes(s.n, s.bs, s.nnzb)
     t = statistics.mean(ms)
-    print(json.dumps({"metric": "ILU0 application (two streamed sweeps) GB/s", "value": nbytes / (t * 1e-3) / 1e9,
+    print(json.dumps({"metric": "ILU0 application (two sweeps) GB/s", "value": nbytes / (t * 1e-3) / 1e9,
                       "unit": "GB/s", "ms_per_apply": t, "steps": args.steps, "warmup": args.warmup,
                       "algorithmic_bytes": nbytes, "peak": peak, "peak_source": kind,
                       "levels": [pc.info()["levels_lower"], pc.info()["levels_upper"]]}), flush=True)
@@ -1015,7 +1015,7 @@ def main():
                        "algorithmic_bytes": ilu_b,
                        "levels": [r["levels"]["levels_lower"], r["levels"]["levels_upper"]]},
         "roofline": {"bound": "hbm",
-                     "kernel": "k_ssweep<8,double> x2 (one ILU0 application: forward + backward streamed sweeps)",
+                     "kernel": "k_wave<8,double> x2 (one ILU0 application: forward + backward lock-step sweeps)",
                      "achieved": ilu_gbs, "peak": r["peak"], "unit": "GB/s", "frac": ilu_gbs / r["peak"],
                      "traffic": traffic, "algorithmic_bytes": ilu_b, "peak_source": r["peak_kind"]},
         "e2e": {"value": r["e2e_s"], "unit": "s", "h2d_bytes_per_step": nnzb * bs * bs * 8 + nnzb * 4

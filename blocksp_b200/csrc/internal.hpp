@@ -77,7 +77,7 @@ struct Workspace {
   DevBuf<DevStatus> status;  // device error word
 };
 
-struct StreamSym;
+struct WaveSym;
 struct FactorPlan;
 
 // Structure-only analysis behind a preconditioner (sorted factor pattern,
@@ -92,8 +92,8 @@ struct SymbolicCache {
   DevBuf<int> f_ptr, f_col, f_diag, order_lo, order_up, task_lo_row, task_lo_len, task_up_row,
       task_up_len, t_ptr, t_row, a_diag;
   DevBuf<int64_t> d_perm, t_blk;
-  // streamed layouts of the two sweeps (block sizes the streamed kernel takes)
-  std::shared_ptr<StreamSym> ss_lo, ss_up;
+  // lock-step layouts of the two sweeps (block sizes their kernel takes)
+  std::shared_ptr<WaveSym> wv_lo, wv_up;
   // elimination plan of the row-resident factorisation kernel
   std::shared_ptr<FactorPlan> plan;
 };

@@ -6,6 +6,7 @@
 //   SOR                  :116-240 -> nu sync-free forward / backward sweeps from x = 0
 //   ILU0::factor         :274-291 -> k_factor mode ILU0 (row-wise, level scheduled)
 //   ILU0::invmul         :294-349 -> unit-L forward sweep + U backward sweep
+//                                    (sweep_wave.cu; here for other block sizes)
 //   IChol0::factor       :393-429 -> k_factor mode ICHOL0
 //   IChol0::invmul       :432-489 -> L forward sweep + L^T backward sweep
 //
@@ -44,7 +45,7 @@
 #include "reduce.cuh"
 #include "sentinel.cuh"
 #include "stage.cuh"
-#include "sweep_stream.hpp"
+#include "sweep_wave.hpp"
 
 namespace bsp {
 
@@ -1021,8 +1022,8 @@ static int sym_transfer(bsp_precond_s* pc, SymbolicCache& C, bool save) {
   BSP_SYM_FIELD(t_blk) BSP_SYM_FIELD(a_diag)
 #undef BSP_SYM_FIELD
   if (save) {
-    C.ss_lo = pc->ss_lo;
-    C.ss_up = pc->ss_up;
+    C.wv_lo = pc->wv_lo;
+    C.wv_up = pc->wv_up;
     C.plan = pc->plan;
     C.h_perm = pc->h_perm;
     C.f_nnzb = pc->f_nnzb;
@@ -1032,8 +1033,8 @@ static int sym_transfer(bsp_precond_s* pc, SymbolicCache& C, bool save) {
     C.n_task_up = pc->n_task_up;
     C.valid = true;
   } else {
-    pc->ss_lo = C.ss_lo;
-    pc->ss_up = C.ss_up;
+    pc->wv_lo = C.wv_lo;
+    pc->wv_up = C.wv_up;
     pc->plan = C.plan;
     pc->h_perm = C.h_perm;
     pc->f_nnzb = C.f_nnzb;
@@ -1309,9 +1310,9 @@ static int analyse_factor_structure(bsp_precond_s* pc, bool lower_only) {
   pc->n_lev_lo = level_order(n, true, lower_deps, order);
   BSP_TRY(upload(pc->order_lo, order));
   BSP_TRY(make_tasks(pc, true, n, lower_deps));
-  // streamed layouts of both sweeps (ILU0: unit L, then U with U_ii^-1;
+  // lock-step layouts of both sweeps (ILU0: unit L, then U with U_ii^-1;
   // IChol0: L with L_ii^-1, then L^T with L_ii^-T)
-  const bool streamed = stream_supported(pc->bs);
+  const bool wave = wave_supported(pc->bs);
   SweepEntries ent;
   // strictly-lower (lower = true) or strictly-upper entries of the factor
   auto tri_entries = [&](bool lower) {
@@ -1327,11 +1328,7 @@ static int analyse_factor_structure(bsp_precond_s* pc, bool lower_only) {
       ent.ptr[i + 1] = (int)ent.col.size();
     }
   };
-  if (streamed) {
-    tri_entries(true);
-    pc->ss_lo = std::make_shared<StreamSym>();
-    BSP_TRY(stream_build(n, true, stream_warps(pc->bs), ent, false, lower_only, false, *pc->ss_lo));
-  }
+  std::vector<int> up_item;  // per row: the item of the backward sweep that reads it
   if (!lower_only) {
     auto upper_deps = [&](int i, auto&& f) {
       for (int e = diag[i] + 1; e < ptr[i + 1]; ++e) f(col[e]);
@@ -1339,10 +1336,10 @@ static int analyse_factor_structure(bsp_precond_s* pc, bool lower_only) {
     pc->n_lev_up = level_order(n, false, upper_deps, order);
     BSP_TRY(upload(pc->order_up, order));
     BSP_TRY(make_tasks(pc, false, n, upper_deps));
-    if (streamed) {
+    if (wave) {
       tri_entries(false);
-      pc->ss_up = std::make_shared<StreamSym>();
-      BSP_TRY(stream_build(n, false, stream_warps(pc->bs), ent, false, true, false, *pc->ss_up));
+      pc->wv_up = std::make_shared<WaveSym>();
+      BSP_TRY(wave_build(n, pc->bs, false, ent, false, true, false, {}, nullptr, &up_item, *pc->wv_up));
     }
   } else {
     // L^T backward: row i depends on rows j > i with L_ji present
@@ -1366,16 +1363,21 @@ static int analyse_factor_structure(bsp_precond_s* pc, bool lower_only) {
     pc->n_lev_up = level_order(n, false, trans_deps, order);
     BSP_TRY(upload(pc->order_up, order));
     BSP_TRY(make_tasks(pc, false, n, trans_deps));
-    if (streamed) {
+    if (wave) {
       ent.ptr = tp;
       ent.col = trow;
       ent.blk = tblk;
-      pc->ss_up = std::make_shared<StreamSym>();
-      BSP_TRY(stream_build(n, false, stream_warps(pc->bs), ent, true, true, true, *pc->ss_up));
+      pc->wv_up = std::make_shared<WaveSym>();
+      BSP_TRY(wave_build(n, pc->bs, false, ent, true, true, true, {}, nullptr, &up_item, *pc->wv_up));
     }
     BSP_TRY(upload(pc->t_ptr, tp));
     BSP_TRY(upload(pc->t_row, trow));
     BSP_TRY(upload(pc->t_blk, tblk));
+  }
+  if (wave) {
+    tri_entries(true);
+    pc->wv_lo = std::make_shared<WaveSym>();
+    BSP_TRY(wave_build(n, pc->bs, true, ent, false, lower_only, false, {}, &up_item, nullptr, *pc->wv_lo));
   }
   return build_factor_plan(pc, n, ptr, col, diag, lower_only);
 }
@@ -1447,9 +1449,9 @@ static int build_diag_inverse(bsp_precond_s* pc) {
                     pc->A->vals.get(), pc->n);
 }
 
-// The factors changed: every streamed copy of them is stale.
-static void stream_invalidate(bsp_precond_s* pc) {
-  for (int k = 0; k < 3; ++k) pc->sv_lo[k].valid = pc->sv_up[k].valid = false;
+// The factors changed: every copy of them in sweep order is stale.
+static void wave_invalidate(bsp_precond_s* pc) {
+  for (int k = 0; k < 3; ++k) pc->vv_lo[k].valid = pc->vv_up[k].valid = false;
 }
 
 static int make_lowp_copies(bsp_precond_s* pc) {
@@ -1478,10 +1480,12 @@ static int make_lowp_copies(bsp_precond_s* pc) {
 
 int precond_build(bsp_precond_s* pc) {
   const int n = pc->n, b2 = pc->bs * pc->bs;
-  stream_invalidate(pc);
+  wave_invalidate(pc);
   BSP_TRY(take(pc->A, pc->dinv, (size_t)std::max(n, 1) * b2));
   BSP_TRY(take(pc->A, pc->flags, std::max(n, 1)));
   BSP_TRY(take(pc->A, pc->ticket, 1));
+  BSP_TRY(pc->wticket.alloc(1));
+  BSP_CUDA_TRY(cudaMemset(pc->wticket.get(), 0, sizeof(unsigned)));
   BSP_CUDA_TRY(cudaMemset(pc->flags.get(), 0, std::max(n, 1) * sizeof(int)));
   switch (pc->kind) {
     case BSP_PC_NONE:
@@ -1545,10 +1549,12 @@ static int relax_offdiag(bsp_precond_s* pc, const double* f0) {
 // from the corrected U_ii / L_ii (general inverses).
 int precond_build_learned(bsp_precond_s* pc, const double* dF) {
   const int n = pc->n, b2 = pc->bs * pc->bs;
-  stream_invalidate(pc);
+  wave_invalidate(pc);
   BSP_TRY(take(pc->A, pc->dinv, (size_t)std::max(n, 1) * b2));
   BSP_TRY(take(pc->A, pc->flags, std::max(n, 1)));
   BSP_TRY(take(pc->A, pc->ticket, 1));
+  BSP_TRY(pc->wticket.alloc(1));
+  BSP_CUDA_TRY(cudaMemset(pc->wticket.get(), 0, sizeof(unsigned)));
   BSP_CUDA_TRY(cudaMemset(pc->flags.get(), 0, std::max(n, 1) * sizeof(int)));
   // LU form on the ILU0 factors; L L^T form on the IChol0 factor (A.lowTri())
   const bool llt = pc->kind == BSP_PC_LEARNED_LLT;
@@ -1595,27 +1601,28 @@ template <typename VT> constexpr int prec_of() {
   return std::is_same<VT, double>::value ? BSP_PREC_F64 : std::is_same<VT, float>::value ? BSP_PREC_F32 : BSP_PREC_BF16;
 }
 
-// z = M^{-1} r through the streamed sweeps (sa: scratch for the forward
-// result).  The stream values of the precision are gathered on first use.
+// z = M^{-1} r through the lock-step sweeps.  The values of the precision are
+// gathered on first use.
 template <typename VT>
-static int apply_streamed(bsp_precond_s* pc, const double* r, double* z, double* sa) {
+static int apply_wave(bsp_precond_s* pc, const double* r, double* z) {
   bsp_handle_s* h = pc->h;
   constexpr int prec = prec_of<VT>();
-  StreamVals& lo = pc->sv_lo[prec];
-  StreamVals& up = pc->sv_up[prec];
-  for (auto* sv : {&lo, &up}) {
-    if (sv->valid) continue;
-    const StreamSym& S = sv == &lo ? *pc->ss_lo : *pc->ss_up;
-    const size_t vb = stream_val_bytes(S, pc->bs, prec), db = stream_dval_bytes(S, pc->bs, prec);
-    if (sv->vals.n < vb) BSP_TRY(take(pc->A, sv->vals, vb));
-    if (db && sv->dvals.n < db) BSP_TRY(take(pc->A, sv->dvals, db));
-    BSP_TRY(stream_gather(h, S, pc->bs, prec, pc->f_vals.get(), pc->dinv.get(), *sv));
+  WaveVals& lo = pc->vv_lo[prec];
+  WaveVals& up = pc->vv_up[prec];
+  for (auto* v : {&lo, &up}) {
+    if (v->valid) continue;
+    const WaveSym& S = v == &lo ? *pc->wv_lo : *pc->wv_up;
+    const size_t vb = wave_val_bytes(S, prec);
+    if (v->vals.n < vb) BSP_TRY(take(pc->A, v->vals, vb));
+    BSP_TRY(wave_gather(h, S, prec, pc->f_vals.get(), pc->dinv.get(), *v));
   }
-  const int64_t nv = (int64_t)pc->n * pc->bs;
-  BSP_TRY(fill_sentinel(h, sa, nv));
-  BSP_TRY(stream_sweep(h, *pc->ss_lo, pc->bs, prec, lo, r, sa, pc->ticket.get()));
-  BSP_TRY(fill_sentinel(h, z, nv));
-  return stream_sweep(h, *pc->ss_up, pc->bs, prec, up, sa, z, pc->ticket.get());
+  const size_t need[2] = {wave_item_values(*pc->wv_up, 1), wave_item_values(*pc->wv_lo, 1)};
+  for (int i = 0; i < 2; ++i)
+    if (pc->s64[i].n < need[i]) BSP_TRY(take(pc->A, pc->s64[i], need[i]));
+  double *w = pc->s64[0].get(), *rp = pc->s64[1].get();
+  BSP_TRY(wave_prepare(h, *pc->wv_lo, *pc->wv_up, r, rp, w, z));
+  BSP_TRY(wave_sweep(h, *pc->wv_lo, prec, lo, rp, w, pc->wticket.get()));
+  return wave_sweep(h, *pc->wv_up, prec, up, w, z, pc->wticket.get());
 }
 
 // z = M^{-1} r (z may alias r).  Every sweep with dependencies writes into a
@@ -1683,10 +1690,7 @@ static int apply_typed(bsp_precond_s* pc, const AT* r, AT* z, const VT* fvals, c
     case BSP_PC_ILU0:
     case BSP_PC_LEARNED_LU: {
       if constexpr (std::is_same<AT, double>::value) {
-        // the streamed sweeps read vectors in 16-byte pieces
-        if (pc->ss_lo && pc->ss_up && reinterpret_cast<uintptr_t>(z) % 16 == 0 &&
-            reinterpret_cast<uintptr_t>(r) % 16 == 0)
-          return apply_streamed<VT>(pc, r, z, sa);
+        if (pc->wv_lo && pc->wv_up) return apply_wave<VT>(pc, r, z);
       }
       p.ptr = pc->f_ptr.get();
       p.idx = pc->f_col.get();
@@ -1713,10 +1717,7 @@ static int apply_typed(bsp_precond_s* pc, const AT* r, AT* z, const VT* fvals, c
     case BSP_PC_ICHOL0:
     case BSP_PC_LEARNED_LLT: {
       if constexpr (std::is_same<AT, double>::value) {
-        // the streamed sweeps read vectors in 16-byte pieces
-        if (pc->ss_lo && pc->ss_up && reinterpret_cast<uintptr_t>(z) % 16 == 0 &&
-            reinterpret_cast<uintptr_t>(r) % 16 == 0)
-          return apply_streamed<VT>(pc, r, z, sa);
+        if (pc->wv_lo && pc->wv_up) return apply_wave<VT>(pc, r, z);
       }
       p.ptr = pc->f_ptr.get();
       p.idx = pc->f_col.get();
@@ -1868,6 +1869,8 @@ int precond_learned_init(bsp_precond_s* pc) {
   BSP_TRY(take(pc->A, pc->dinv, (size_t)std::max(n, 1) * b2));
   BSP_TRY(take(pc->A, pc->flags, std::max(n, 1)));
   BSP_TRY(take(pc->A, pc->ticket, 1));
+  BSP_TRY(pc->wticket.alloc(1));
+  BSP_CUDA_TRY(cudaMemset(pc->wticket.get(), 0, sizeof(unsigned)));
   BSP_CUDA_TRY(cudaMemset(pc->flags.get(), 0, std::max(n, 1) * sizeof(int)));
   return build_factor_structure(pc, pc->kind == BSP_PC_LEARNED_LLT);
 }
@@ -1877,7 +1880,7 @@ int precond_learned_init(bsp_precond_s* pc) {
 // (both built on the same matrix) and gets fresh diagonal inverses.
 int precond_learned_refresh(bsp_precond_s* work, const bsp_precond_s* ilu, const double* dF) {
   if (work->f_nnzb != ilu->f_nnzb || work->n != ilu->n || work->bs != ilu->bs) return BSP_INVALID;
-  stream_invalidate(work);
+  wave_invalidate(work);
   const int b2 = work->bs * work->bs;
   const int64_t tot = work->f_nnzb * b2;
   if (tot > 0)
@@ -2016,8 +2019,8 @@ int bsp_precond_destroy(bsp_precond_t pc) {
     for (int i = 0; i < 3; ++i) {
       give(A, pc->s64[i]);
       give(A, pc->s32[i]);
-      give(A, pc->sv_lo[i].vals); give(A, pc->sv_lo[i].dvals);
-      give(A, pc->sv_up[i].vals); give(A, pc->sv_up[i].dvals);
+      give(A, pc->vv_lo[i].vals);
+      give(A, pc->vv_up[i].vals);
     }
   }
   delete pc;

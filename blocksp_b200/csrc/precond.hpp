@@ -2,7 +2,7 @@
 // single-system, batched and learned solvers).
 #pragma once
 #include "internal.hpp"
-#include "sweep_stream.hpp"
+#include "sweep_wave.hpp"
 
 namespace bsp {
 // Elimination plan of a block ILU0 / IChol0 factorisation (pattern only).
@@ -68,12 +68,13 @@ struct bsp_precond_s {
   // iterates and the copy of an in-place right-hand side
   bsp::DevBuf<double> s64[3];
   bsp::DevBuf<float> s32[3];
-  // streamed sweeps (ILU0 / IChol0 and the learned factors, FP64 vectors):
+  // lock-step sweeps (ILU0 / IChol0 and the learned factors, FP64 vectors):
   // the layout, shared with the matrix's symbolic cache, and its values per
   // precision (index BSP_PREC_*), gathered from f_vals / dinv on first use
   // after every change of the factors
-  std::shared_ptr<bsp::StreamSym> ss_lo, ss_up;
-  bsp::StreamVals sv_lo[3], sv_up[3];
+  std::shared_ptr<bsp::WaveSym> wv_lo, wv_up;
+  bsp::WaveVals vv_lo[3], vv_up[3];
+  bsp::DevBuf<unsigned> wticket;  // 0 between sweeps (every sweep resets it)
   // elimination plan of the factorisation (shared with the matrix's cache)
   std::shared_ptr<bsp::FactorPlan> plan;
 };

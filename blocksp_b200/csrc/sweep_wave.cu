@@ -1,0 +1,255 @@
+// sweep_wave.cu — building, filling and launching the lock-step sweeps.
+//
+// Reference: blocksp_preconditioners.hpp:294-349 (ILU0::invmul: unit-L
+// forward substitution, then backward substitution with D_Inv[i] = U_ii^-1)
+// and :432-489 (IChol0::invmul: L forward with L_ii^-1, then L^T backward
+// through the column structure of L with L_ii^-T).  Natural order is kept.
+#include "sweep_wave.cuh"
+
+namespace bsp {
+
+int grid_for(const bsp_handle_s* h, int64_t n, int threads);
+
+#define BSP_WAVE_SIZES(X) X(1) X(2) X(3) X(4) X(5) X(6) X(8) X(16)
+
+bool wave_supported(int bs) {
+  switch (bs) {
+#define BSP_WAVE_CASE(B) case B:
+    BSP_WAVE_SIZES(BSP_WAVE_CASE)
+#undef BSP_WAVE_CASE
+    return true;
+    default: return false;
+  }
+}
+
+WaveShape wave_shape(int bs) {
+  WaveShape s;
+  switch (bs) {
+#define BSP_WAVE_CASE(B) \
+  case B: s = wave_shape_of<B>(); break;
+    BSP_WAVE_SIZES(BSP_WAVE_CASE)
+#undef BSP_WAVE_CASE
+    default: break;
+  }
+  return s;
+}
+
+// ------------------------------------------------------------------ values
+// Stored block b: minus factor block blk_src[b] (transposed when trans),
+// premultiplied by its row's D when the sweep has D blocks, or what the
+// negative codes of wave_plan.h say.
+template <int BS, typename VT, bool HAS_D>
+__global__ void k_wave_gather(int64_t nblk, const int64_t* __restrict__ blk_src, const int* __restrict__ blk_row,
+                              const double* __restrict__ src, const double* __restrict__ dinv, int trans, int trans_d,
+                              VT* __restrict__ dst) {
+  constexpr int B2 = BS * BS;
+  const int64_t total = nblk * B2;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t b = t / B2;
+    const int k = (int)(t - b * B2);
+    const int a = WaveDim<BS>::kChunk ? k / BS : k % BS, c = WaveDim<BS>::kChunk ? k % BS : k / BS;
+    const int64_t sb = blk_src[b];
+    double v = 0.0;
+    if (sb >= 0) {
+      const double* B = src + sb * B2;
+      if constexpr (HAS_D) {
+        const double* D = dinv + (int64_t)blk_row[b] * B2;
+#pragma unroll
+        for (int m = 0; m < BS; ++m)
+          v = fma(trans_d ? D[m * BS + a] : D[a * BS + m], trans ? B[c * BS + m] : B[m * BS + c], v);
+      } else {
+        v = trans ? B[c * BS + a] : B[a * BS + c];
+      }
+      v = -v;
+    } else if (sb == kWaveD) {
+      v = dinv[(int64_t)blk_row[b] * B2 + (trans_d ? c * BS + a : a * BS + c)];
+    } else if (sb == kWaveOne) {
+      v = a == c ? 1.0 : 0.0;
+    }
+    if constexpr (sizeof(VT) == 8) dst[t] = v;
+    else if constexpr (sizeof(VT) == 4) dst[t] = (float)v;
+    else dst[t] = __float2bfloat16_rn((float)v);
+  }
+}
+
+template <int BS, typename VT>
+static int gather_t(bsp_handle_s* h, const WaveSym& S, const double* fvals, const double* dinv, WaveVals& out) {
+  const int g = grid_for(h, S.n_blk * BS * BS, 256);
+  VT* dst = reinterpret_cast<VT*>(out.vals.get());
+  count_launch();
+  if (S.has_d)
+    k_wave_gather<BS, VT, true><<<g, 256, 0, h->stream>>>(S.n_blk, S.blk_src.get(), S.blk_row.get(), fvals, dinv,
+                                                          S.trans_blocks, S.trans_d, dst);
+  else
+    k_wave_gather<BS, VT, false><<<g, 256, 0, h->stream>>>(S.n_blk, S.blk_src.get(), S.blk_row.get(), fvals, dinv,
+                                                           S.trans_blocks, S.trans_d, dst);
+  BSP_CUDA_TRY(cudaPeekAtLastError());
+  return BSP_OK;
+}
+
+static size_t prec_bytes(int prec) { return prec == BSP_PREC_F64 ? 8 : prec == BSP_PREC_F32 ? 4 : 2; }
+size_t wave_val_bytes(const WaveSym& S, int prec) {
+  // W items past the last one are read (and dropped)
+  return (size_t)(S.n_blk + (int64_t)wave_shape(S.bs).W * (S.ne + 1)) * S.bs * S.bs * prec_bytes(prec);
+}
+
+int wave_gather(bsp_handle_s* h, const WaveSym& S, int prec, const double* fvals, const double* dinv, WaveVals& out) {
+  const size_t vb = wave_val_bytes(S, prec);
+  if (out.vals.n < vb) BSP_TRY(out.vals.alloc(vb));
+  if (S.n_blk > 0) {
+    int st = BSP_INVALID;
+    switch (S.bs) {
+#define BSP_WAVE_CASE(B)                                                                      \
+  case B:                                                                                     \
+    st = prec == BSP_PREC_F64   ? gather_t<B, double>(h, S, fvals, dinv, out)                 \
+         : prec == BSP_PREC_F32 ? gather_t<B, float>(h, S, fvals, dinv, out)                  \
+                                : gather_t<B, __nv_bfloat16>(h, S, fvals, dinv, out);         \
+    break;
+      BSP_WAVE_SIZES(BSP_WAVE_CASE)
+#undef BSP_WAVE_CASE
+      default: break;
+    }
+    BSP_TRY(st);
+  }
+  out.valid = true;
+  return BSP_OK;
+}
+
+// ------------------------------------------------------------------ build
+template <typename T, typename H> static int upload_as(DevBuf<T>& d, const std::vector<H>& v) {
+  static_assert(sizeof(T) == sizeof(H), "same layout on host and device");
+  BSP_TRY(d.alloc(v.empty() ? 1 : v.size()));
+  if (!v.empty()) BSP_CUDA_TRY(cudaMemcpy(d.get(), v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+  return BSP_OK;
+}
+
+int wave_build(int n, int bs, bool ascending, const SweepEntries& ent, bool trans_blocks, bool has_d, bool trans_d,
+               const std::vector<int>& group_beg, const std::vector<int>* row_item, std::vector<int>* item_of,
+               WaveSym& S) {
+  WavePlan P;
+  if (!wave_plan(n, ascending, wave_shape(bs), has_d, ent, group_beg, P)) {
+    record_error("triangular sweep: the dependencies are not triangular, or the stream is too long");
+    return BSP_INVALID;
+  }
+  if (item_of) {
+    item_of->assign(n, 0);
+    for (size_t i = 0; i < P.item_row.size(); ++i)
+      if (P.item_row[i] >= 0) (*item_of)[P.item_row[i]] = (int)i;
+  }
+  if (row_item) {
+    for (auto& r : P.rec)
+      if (r.row >= 0) r.row = (*row_item)[r.row];
+    for (int& r : P.ext_row) r = (*row_item)[r];
+  }
+  S.n = n;
+  S.bs = bs;
+  S.n_item = (int64_t)P.rec.size();
+  S.to_items = row_item != nullptr;
+  S.n_super = P.n_super;
+  S.n_levels = P.n_levels;
+  S.ne = P.ne;
+  S.n_blk = (int64_t)P.blk_src.size();
+  S.trans_blocks = trans_blocks;
+  S.has_d = has_d;
+  S.trans_d = trans_d;
+  BSP_TRY(upload_as(S.super_step, P.super_step));
+  BSP_TRY(upload_as(S.super_group, P.super_group));
+  BSP_TRY(upload_as(S.step, P.step));
+  BSP_TRY(upload_as(S.rec, P.rec));
+  BSP_TRY(upload_as(S.item_row, P.item_row));
+  BSP_TRY(upload_as(S.ext_row, P.ext_row));
+  BSP_TRY(upload_as(S.blk_src, P.blk_src));
+  BSP_TRY(upload_as(S.blk_row, P.blk_row));
+  return BSP_OK;
+}
+
+// ------------------------------------------------------------------ sweep
+size_t wave_item_values(const WaveSym& S, int nrhs) {
+  return (size_t)std::max<int64_t>(S.n_item, 1) * wave_ld_of(nrhs * S.bs);
+}
+
+// rp = r in item order and z's sentinel (a row is read and replaced by the same
+// thread, so z may alias r); w's sentinel.
+template <int BS>
+__global__ void k_wave_prepare(int64_t n_item, const int* __restrict__ item_row, const double* r, double* rp,
+                               double* z, int64_t n_w, unsigned long long* __restrict__ w) {
+  constexpr int LD = wave_ld_of(BS);
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x, t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (int64_t t = t0; t < n_item * BS; t += stride) {
+    const int64_t i = t / BS;
+    const int c = (int)(t - i * BS), row = __ldg(item_row + i);
+    if (row >= 0) {
+      const int64_t k = (int64_t)row * BS + c;
+      rp[i * LD + c] = r[k];
+      reinterpret_cast<unsigned long long*>(z)[k] = kSentinel64;
+    }
+  }
+  for (int64_t t = t0; t < n_w; t += stride) w[t] = kSentinel64;
+}
+
+int wave_prepare(bsp_handle_s* h, const WaveSym& lo, const WaveSym& up, const double* r, double* rp, double* w,
+                 double* z) {
+  const int64_t nw = (int64_t)wave_item_values(up, 1);
+  const int g = grid_for(h, std::max(lo.n_item * lo.bs, nw), 256);
+  auto* ws = reinterpret_cast<unsigned long long*>(w);
+  count_launch();
+  switch (lo.bs) {
+#define BSP_WAVE_CASE(B)                                                                          \
+  case B:                                                                                         \
+    k_wave_prepare<B><<<g, 256, 0, h->stream>>>(lo.n_item, lo.item_row.get(), r, rp, z, nw, ws);  \
+    break;
+    BSP_WAVE_SIZES(BSP_WAVE_CASE)
+#undef BSP_WAVE_CASE
+    default: return BSP_INVALID;
+  }
+  BSP_CUDA_TRY(cudaPeekAtLastError());
+  return BSP_OK;
+}
+
+template <int BS, typename VT>
+static int sweep_t(bsp_handle_s* h, const WaveSym& S, const WaveP<VT>& p) {
+  if (S.ne == 2) return S.has_d ? wave_launch<BS, VT, true, 2, 1>(h, p) : wave_launch<BS, VT, false, 2, 1>(h, p);
+  return S.has_d ? wave_launch<BS, VT, true, 3, 1>(h, p) : wave_launch<BS, VT, false, 3, 1>(h, p);
+}
+
+template <typename VT>
+static int sweep_typed(bsp_handle_s* h, const WaveSym& S, const WaveVals& V, const double* rhs, double* x,
+                       unsigned* ticket) {
+  WaveP<VT> p{};
+  p.n_super = S.n_super;
+  p.super_step = S.super_step.get();
+  p.super_group = S.super_group.get();
+  p.step = S.step.get();
+  p.rec = S.rec.get();
+  p.ext_row = S.ext_row.get();
+  p.vals = reinterpret_cast<const VT*>(V.vals.get());
+  p.rhs = rhs;
+  p.x = x;
+  p.xs = S.to_items ? wave_ld_of(S.bs) : S.bs;
+  p.spin_limit = h->spin_limit;
+  p.ticket = ticket;
+  p.st = h->ws.status.get();
+  switch (S.bs) {
+#define BSP_WAVE_CASE(B) \
+  case B: return sweep_t<B, VT>(h, S, p);
+    BSP_WAVE_SIZES(BSP_WAVE_CASE)
+#undef BSP_WAVE_CASE
+    default: break;
+  }
+  record_error("triangular sweep: unsupported block size");
+  return BSP_INVALID;
+}
+
+int wave_sweep(bsp_handle_s* h, const WaveSym& S, int prec, const WaveVals& V, const double* rhs, double* x,
+               unsigned* ticket) {
+  if (!V.valid) {
+    record_error("triangular sweep: values not gathered");
+    return BSP_INVALID;
+  }
+  if (S.n_super == 0) return BSP_OK;
+  if (prec == BSP_PREC_F64) return sweep_typed<double>(h, S, V, rhs, x, ticket);
+  if (prec == BSP_PREC_F32) return sweep_typed<float>(h, S, V, rhs, x, ticket);
+  return sweep_typed<__nv_bfloat16>(h, S, V, rhs, x, ticket);
+}
+
+}  // namespace bsp
