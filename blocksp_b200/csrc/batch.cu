@@ -13,9 +13,9 @@
 // Design:
 //   * systems of the same block size form a group, stored as ONE block-diagonal
 //     BSR matrix (systems concatenated); IChol0 of a block-diagonal matrix is
-//     the block-diagonal of the per-system factors, so the existing level /
-//     chain analysis and factorisation run once over the whole group, and the
-//     sync-free sweeps run every system's chains in the same persistent launch;
+//     the block-diagonal of the per-system factors, so the factorisation runs
+//     once over the whole group, and the lock-step sweeps (sweep_wave.cuh) run
+//     the super-tasks of every system in one launch, a system's own plan each;
 //   * right-hand sides are interleaved per block row (the solArray<T,bs,R>
 //     layout), so each matrix / factor block is read once for all R of them;
 //   * per-pair scalars come from segmented reductions over fixed 64-row tiles
@@ -28,9 +28,9 @@
 //     of the same iteration graph is kept as the alternative mode);
 //   * converged systems drop out: every tile, task and reduction of a system
 //     whose pairs are all finished is skipped;
-//   * launch shapes (threads per CTA and CTAs per SM of the tile kernels, CTAs
-//     per SM of the sweeps) are chosen per group by timing the candidates on
-//     the group's own data the first time it is solved (an autotuner).
+//   * launch shapes (threads per CTA and CTAs per SM of the tile kernels) are
+//     chosen per group by timing the candidates on the group's own data the
+//     first time it is solved (an autotuner).
 #include <algorithm>
 #include <chrono>
 #include <cstring>
@@ -69,9 +69,10 @@ struct BGroupP {
   const int* col_idx;
   const double* vals;
   double *x, *r, *z, *w, *p, *q, *part0, *part1;
+  double* rp;               // r in the forward sweep's item order
+  const int *item_lo, *item_up;  // per row: its item of the forward / backward sweep
   BState* st;
   int* sys_active;
-  unsigned* tickets;        // [0] forward sweep, [1] backward sweep
   double* hist;
   int hist_cap;
   const BOpts* opts;
@@ -208,8 +209,15 @@ template <int R> __device__ __forceinline__ void store_partials(double* part, in
   }
 }
 
-// x += alpha p, r -= alpha q for running pairs; part1 = r . r; the sweep
-// outputs w, z of the tile are re-filled with the sentinel.
+// Row e / (R BS) of element e of a vector, as its place in the order of items.
+template <int BS, int R> __device__ __forceinline__ int64_t item_place(const int* item, int64_t e) {
+  const int64_t row = e / (R * BS);
+  return (int64_t)__ldg(item + row) * (R * BS) + (e - row * (R * BS));
+}
+
+// x += alpha p, r -= alpha q for running pairs; part1 = r . r; r goes to the
+// forward sweep's item order too, and the sweep outputs w (in the backward
+// sweep's item order) and z of the tile are re-filled with the sentinel.
 template <int BS, int R>
 __global__ void __launch_bounds__(kBatchMaxThreads) k_bt_update(const BGroupP g) {
   BT_FOR_TILES(g, t) {
@@ -235,7 +243,8 @@ __global__ void __launch_bounds__(kBatchMaxThreads) k_bt_update(const BGroupP g)
       const double sq = rv * rv;
 #pragma unroll
       for (int k = 0; k < R; ++k) acc[k] += (k == rhs) ? sq : 0.0;
-      reinterpret_cast<unsigned long long*>(g.w)[e] = kSentinel64;
+      g.rp[item_place<BS, R>(g.item_lo, e)] = rv;
+      reinterpret_cast<unsigned long long*>(g.w)[item_place<BS, R>(g.item_up, e)] = kSentinel64;
       reinterpret_cast<unsigned long long*>(g.z)[e] = kSentinel64;
     }
     store_partials<R>(g.part1, t, acc);
@@ -293,7 +302,8 @@ __global__ void __launch_bounds__(kBatchMaxThreads) k_bt_init(const BGroupP g) {
     BT_FOR_ELEMS(e, rhs, r0, r1) {
       (void)rhs;
       g.x[e] = 0.0;
-      reinterpret_cast<unsigned long long*>(g.w)[e] = kSentinel64;
+      g.rp[item_place<BS, R>(g.item_lo, e)] = g.r[e];
+      reinterpret_cast<unsigned long long*>(g.w)[item_place<BS, R>(g.item_up, e)] = kSentinel64;
       reinterpret_cast<unsigned long long*>(g.z)[e] = kSentinel64;
     }
   }
@@ -333,7 +343,6 @@ template <int R, int MODE>
 __global__ void k_bt_fin(const BGroupP g) {
   const int s = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
-  if (MODE == FIN_RES && blockIdx.x == 0 && threadIdx.x < 2) g.tickets[threadIdx.x] = 0u;
   if (s >= g.n_sys) return;
   if (MODE != FIN_INIT && !g.sys_active[s]) return;
   const int t0 = g.sys_tile[s], t1 = g.sys_tile[s + 1];
@@ -436,297 +445,6 @@ __global__ void k_bt_copy(int n_sys, const int64_t* __restrict__ user_off, const
   }
 }
 
-// ------------------------------------------------------------------ sweeps
-// Multi-RHS sync-free IChol0 sweeps over the chains of every active system.
-// TRANS = false: w_i = L_ii^-1 (r_i - sum_{j<i} L_ij w_j)      (forward, L by rows)
-// TRANS = true:  z_i = L_ii^-T (w_i - sum_{j>i} L_ji^T z_j)    (backward, L by columns)
-// (blocksp_preconditioners.hpp:432-489, per RHS.)
-struct BSweepP {
-  int n_tasks;
-  const int* task_row;
-  const int* task_len;
-  const int* task_sys;
-  int task_dir;
-  const int* sys_active;
-  const int* ptr;
-  const int* idx;
-  const int64_t* blk;  // null: entry index
-  const int* diag;     // forward: entries [ptr[i], diag[i])
-  const double* vals;
-  const double* dinv;
-  const double* rhs;
-  double* x;
-  unsigned* ticket;
-  DevStatus* st;
-  unsigned spin_limit;  // polls before a wait gives up with BSP_TIMEOUT
-};
-
-constexpr int kBSweepThreads = 256;
-
-template <int BS, int R, bool TRANS>
-__global__ void __launch_bounds__(kBSweepThreads) k_bt_sweep(const BSweepP p) {
-  using M = BlockMap<BS, double>;
-  using CV = typename Chunk<double>::vec;
-  constexpr int V = M::V, G = M::G, P = M::P, CPR = M::CPR, RPP = M::RPP, CPB = M::CPB;
-  constexpr int GPC = kBSweepThreads / G;
-  constexpr int LD = R * BS;
-  // dependency entries whose blocks are loaded ahead: fewer with more RHS,
-  // whose x values take the registers
-  constexpr int NPF = (P == 1) ? (R >= 4 ? 2 : 4) : (P == 2 && R < 4 ? 2 : 1);
-  constexpr int XV = TRANS ? P : V;
-  __shared__ double sm_s[GPC][LD];
-  __shared__ double sm_x[GPC][LD];
-  const int gl = threadIdx.x % G;
-  const int gid = threadIdx.x / G;
-  const int lane = threadIdx.x & 31;
-  const int gbase = lane - gl;
-  const unsigned gmask = (G == 32) ? 0xffffffffu : (((1u << G) - 1u) << gbase);
-  const int c0 = (gl % CPR) * V;
-  const CV* vb = reinterpret_cast<const CV*>(p.vals);
-  double* s = sm_s[gid];
-  double* xs = sm_x[gid];
-  while (true) {
-    int t = 0;
-    if (gl == 0) t = (int)atomicAdd(p.ticket, 1u);
-    t = __shfl_sync(gmask, t, gbase);
-    if (t >= p.n_tasks) break;
-    if (!p.sys_active[__ldg(p.task_sys + t)]) continue;
-    const int i0 = __ldg(p.task_row + t);
-    const int len = __ldg(p.task_len + t);
-    CV nf[NPF][P], nd[P];
-    int nbeg, nend;
-    auto range = [&](int r, int& b0, int& b1) {
-      b0 = __ldg(p.ptr + r);
-      b1 = TRANS ? __ldg(p.ptr + r + 1) : __ldg(p.diag + r);
-    };
-    auto prefetch = [&](int r, int& b0, int& b1) {
-      range(r, b0, b1);
-#pragma unroll
-      for (int u = 0; u < NPF; ++u) {
-        if (b0 + u < b1) {
-          const int64_t b = p.blk ? __ldg(p.blk + b0 + u) : (int64_t)(b0 + u);
-#pragma unroll
-          for (int q = 0; q < P; ++q) nf[u][q] = ld_stream(vb + b * CPB + q * G + gl);
-        }
-      }
-      const CV* db = reinterpret_cast<const CV*>(p.dinv) + (int64_t)r * CPB;
-#pragma unroll
-      for (int q = 0; q < P; ++q) nd[q] = ld_stream(db + q * G + gl);
-    };
-    prefetch(i0, nbeg, nend);
-    for (int step = 0; step < len; ++step) {
-      const int i = i0 + step * p.task_dir;
-      const int prev = step > 0 ? i - p.task_dir : -1;
-      const int beg = nbeg, end = nend;
-      CV pf[NPF][P], pd[P];
-#pragma unroll
-      for (int u = 0; u < NPF; ++u)
-#pragma unroll
-        for (int q = 0; q < P; ++q) pf[u][q] = nf[u][q];
-#pragma unroll
-      for (int q = 0; q < P; ++q) pd[q] = nd[q];
-      if (step + 1 < len) prefetch(i + p.task_dir, nbeg, nend);
-      double acc[P][R];   // forward: per block row q and RHS
-      double tac[R][V];   // backward: per RHS and column
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-#pragma unroll
-        for (int q = 0; q < P; ++q) acc[q][r] = 0.0;
-#pragma unroll
-        for (int v = 0; v < V; ++v) tac[r][v] = 0.0;
-      }
-      // x values of dependency j for every RHS: from shared memory when j is
-      // the chain's previous row, else from global memory (polled)
-      auto load_x = [&](bool from_prev, int j, double (&xv)[R][XV]) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          if constexpr (!TRANS) {
-            if (from_prev) {
-#pragma unroll
-              for (int v = 0; v < V; ++v) xv[r][v] = xs[r * BS + c0 + v];
-            } else {
-              ld_vec_cg<V>(p.x + (int64_t)j * LD + r * BS + c0, xv[r]);
-            }
-          } else {
-#pragma unroll
-            for (int q = 0; q < P; ++q) {
-              const int rr = q * RPP + gl / CPR;
-              xv[r][q] = from_prev ? xs[r * BS + rr] : __ldcg(p.x + (int64_t)j * LD + r * BS + rr);
-            }
-          }
-        }
-      };
-      auto poll_x = [&](int j, double (&xv)[R][XV]) {
-        bool pending = false;
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-#pragma unroll
-          for (int v = 0; v < XV; ++v) pending |= is_sentinel(xv[r][v]);
-        unsigned spins = 0;
-        while (pending) {
-          poll_pause(spins);
-          pending = false;
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-#pragma unroll
-            for (int v = 0; v < XV; ++v) {
-              const int64_t k = TRANS ? (int64_t)j * LD + r * BS + v * RPP + gl / CPR
-                                      : (int64_t)j * LD + r * BS + c0 + v;
-              xv[r][v] = ld_poll(p.x + k);
-              pending |= is_sentinel(xv[r][v]);
-            }
-          }
-          if (pending) {
-            if (++spins > p.spin_limit) {
-              set_status(p.st, BSP_TIMEOUT, i);
-              break;
-            }
-            if ((spins & 255u) == 0u && *reinterpret_cast<volatile int*>(&p.st->code) != 0) break;
-          }
-        }
-      };
-      auto fma_entry = [&](const CV (&a)[P], const double (&xv)[R][XV]) {
-#pragma unroll
-        for (int q = 0; q < P; ++q) {
-          double av[V];
-          unpack(a[q], av);
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            if constexpr (!TRANS) {
-#pragma unroll
-              for (int v = 0; v < V; ++v) acc[q][r] = fma(av[v], xv[r][v], acc[q][r]);
-            } else {
-#pragma unroll
-              for (int v = 0; v < V; ++v) tac[r][v] = fma(av[v], xv[r][q], tac[r][v]);
-            }
-          }
-        }
-      };
-      {
-        double xv[NPF][R][XV];
-        int jj[NPF];
-        bool has[NPF];
-#pragma unroll
-        for (int u = 0; u < NPF; ++u) {
-          has[u] = beg + u < end;
-          if (has[u]) {
-            jj[u] = __ldg(p.idx + beg + u);
-            load_x(jj[u] == prev, jj[u], xv[u]);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < NPF; ++u) {
-          if (has[u]) {
-            if (jj[u] != prev) poll_x(jj[u], xv[u]);
-            fma_entry(pf[u], xv[u]);
-          }
-        }
-      }
-      for (int e = beg + NPF; e < end; ++e) {
-        const int j = __ldg(p.idx + e);
-        const int64_t b = p.blk ? __ldg(p.blk + e) : (int64_t)e;
-        CV a[P];
-#pragma unroll
-        for (int q = 0; q < P; ++q) a[q] = ld_stream(vb + b * CPB + q * G + gl);
-        double xv[R][XV];
-        load_x(j == prev, j, xv);
-        if (j != prev) poll_x(j, xv);
-        fma_entry(a, xv);
-      }
-      // s = rhs_i - sum
-      if constexpr (!TRANS) {
-#pragma unroll
-        for (int q = 0; q < P; ++q)
-#pragma unroll
-          for (int r = 0; r < R; ++r) acc[q][r] = row_reduce<CPR>(acc[q][r], gmask);
-        if (gl % CPR == 0) {
-#pragma unroll
-          for (int q = 0; q < P; ++q) {
-            const int rr = q * RPP + gl / CPR;
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-              s[r * BS + rr] = __ldcg(p.rhs + (int64_t)i * LD + r * BS + rr) - acc[q][r];
-          }
-        }
-      } else {
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-#pragma unroll
-          for (int v = 0; v < V; ++v)
-#pragma unroll
-            for (int o = CPR; o < G; o <<= 1) tac[r][v] += __shfl_xor_sync(gmask, tac[r][v], o);
-        if (gl < CPR) {
-#pragma unroll
-          for (int r = 0; r < R; ++r)
-#pragma unroll
-            for (int v = 0; v < V; ++v)
-              s[r * BS + c0 + v] = __ldcg(p.rhs + (int64_t)i * LD + r * BS + c0 + v) - tac[r][v];
-        }
-      }
-      __syncwarp(gmask);
-      if constexpr (!TRANS) {
-        // x_i = L_ii^-1 s: lane holds Dinv[row q][c0..c0+V)
-#pragma unroll
-        for (int q = 0; q < P; ++q) {
-          double av[V];
-          unpack(pd[q], av);
-          double o[R];
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            o[r] = 0.0;
-#pragma unroll
-            for (int v = 0; v < V; ++v) o[r] = fma(av[v], s[r * BS + c0 + v], o[r]);
-            o[r] = row_reduce<CPR>(o[r], gmask);
-          }
-          if (gl % CPR == 0) {
-            const int rr = q * RPP + gl / CPR;
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-              p.x[(int64_t)i * LD + r * BS + rr] = o[r];
-              xs[r * BS + rr] = o[r];
-            }
-          }
-        }
-      } else {
-        // x_i = L_ii^-T s: lane holds Dinv[rr][c0..c0+V) and adds Dinv[rr][c] s[rr]
-        double o[R][V];
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-#pragma unroll
-          for (int v = 0; v < V; ++v) o[r][v] = 0.0;
-#pragma unroll
-        for (int q = 0; q < P; ++q) {
-          const int rr = q * RPP + gl / CPR;
-          double av[V];
-          unpack(pd[q], av);
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            const double sr = s[r * BS + rr];
-#pragma unroll
-            for (int v = 0; v < V; ++v) o[r][v] = fma(av[v], sr, o[r][v]);
-          }
-        }
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-#pragma unroll
-          for (int v = 0; v < V; ++v)
-#pragma unroll
-            for (int off = CPR; off < G; off <<= 1) o[r][v] += __shfl_xor_sync(gmask, o[r][v], off);
-        if (gl < CPR) {
-#pragma unroll
-          for (int r = 0; r < R; ++r)
-#pragma unroll
-            for (int v = 0; v < V; ++v) {
-              p.x[(int64_t)i * LD + r * BS + c0 + v] = o[r][v];
-              xs[r * BS + c0 + v] = o[r][v];
-            }
-        }
-      }
-      __syncwarp(gmask);
-    }
-  }
-}
-
 }  // namespace bsp
 
 // ================================================================= host side
@@ -736,7 +454,7 @@ namespace {
 
 struct TuneCfg {
   int threads = 256, ctas_per_sm = 2;   // tile kernels
-  int sweep_ctas_per_sm = 0;            // 0: occupancy maximum
+  int sweep_ctas_per_sm = 1;            // the sweeps run one CTA per SM
 };
 
 struct BatchGroup {
@@ -746,11 +464,15 @@ struct BatchGroup {
   bsp_matrix_t A = nullptr;
   bsp_precond_t pc = nullptr;
   int n_tiles = 0;
-  DevBuf<int> tile_sys, tile_row, sys_tile, task_sys_lo, task_sys_up;
+  DevBuf<int> tile_sys, tile_row, sys_tile;
   DevBuf<int64_t> sys_row, user_off;
   // per-solve state for R right-hand sides
   int R = 0, hist_cap = 0;
-  DevBuf<double> x, r, z, w, p, q, part0, part1, hist;
+  // the two sweeps for this R (super-tasks stay inside a system)
+  WaveSym lo, up;
+  WaveVals v_lo, v_up;
+  DevBuf<int> item_lo, item_up;
+  DevBuf<double> x, r, rp, z, w, p, q, part0, part1, hist;
   DevBuf<BState> st;
   DevBuf<int> sys_active;
   DevBuf<unsigned> tickets;
@@ -819,49 +541,13 @@ BGroupP view(bsp_batch_s* B, BatchGroup& g) {
   v.part1 = g.part1.get();
   v.st = g.st.get();
   v.sys_active = g.sys_active.get();
-  v.tickets = g.tickets.get();
+  v.rp = g.rp.get();
+  v.item_lo = g.item_lo.get();
+  v.item_up = g.item_up.get();
   v.hist = g.hist_cap > 0 ? g.hist.get() : nullptr;
   v.hist_cap = g.hist_cap;
   v.opts = B->opts.get();
   return v;
-}
-
-BSweepP sweep_params(bsp_batch_s* B, BatchGroup& g, bool fwd) {
-  bsp_precond_s* pc = g.pc;
-  BSweepP p{};
-  p.sys_active = g.sys_active.get();
-  p.dinv = pc->dinv.get();
-  p.vals = pc->f_vals.get();
-  p.st = B->h->ws.status.get();
-  p.spin_limit = B->h->spin_limit;
-  if (fwd) {
-    p.n_tasks = pc->n_task_lo;
-    p.task_row = pc->task_lo_row.get();
-    p.task_len = pc->task_lo_len.get();
-    p.task_sys = g.task_sys_lo.get();
-    p.task_dir = 1;
-    p.ptr = pc->f_ptr.get();
-    p.idx = pc->f_col.get();
-    p.diag = pc->f_diag.get();
-    p.blk = nullptr;
-    p.rhs = g.r.get();
-    p.x = g.w.get();
-    p.ticket = g.tickets.get();
-  } else {
-    p.n_tasks = pc->n_task_up;
-    p.task_row = pc->task_up_row.get();
-    p.task_len = pc->task_up_len.get();
-    p.task_sys = g.task_sys_up.get();
-    p.task_dir = -1;
-    p.ptr = pc->t_ptr.get();
-    p.idx = pc->t_row.get();
-    p.blk = pc->t_blk.get();
-    p.diag = nullptr;
-    p.rhs = g.w.get();
-    p.x = g.z.get();
-    p.ticket = g.tickets.get() + 1;
-  }
-  return p;
 }
 
 // Kernel set of one (block size, R) instantiation.
@@ -876,15 +562,13 @@ struct Kernels {
   void (*fin_alpha)(const BGroupP);
   void (*fin_res)(const BGroupP);
   void (*fin_beta)(const BGroupP);
-  void (*sweep_fwd)(const BSweepP);
-  void (*sweep_bwd)(const BSweepP);
 };
 
 template <int BS, int R> Kernels kernels_t() {
   return Kernels{k_bt_spmv<BS, R>,        k_bt_update<BS, R>,      k_bt_dot_rz<BS, R>,
                  k_bt_pupd<BS, R>,        k_bt_init<BS, R>,        k_bt_init_dots<BS, R>,
                  k_bt_fin<R, FIN_INIT>,   k_bt_fin<R, FIN_ALPHA>,  k_bt_fin<R, FIN_RES>,
-                 k_bt_fin<R, FIN_BETA>,   k_bt_sweep<BS, R, false>, k_bt_sweep<BS, R, true>};
+                 k_bt_fin<R, FIN_BETA>};
 }
 
 template <int BS> bool kernels_r(int R, Kernels& k) {
@@ -905,43 +589,37 @@ bool kernels_for(int bs, int R, Kernels& k) {
   }
 }
 
-int sweep_grid(bsp_batch_s* B, BatchGroup& g, void (*kern)(const BSweepP)) {
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBSweepThreads, 0) != cudaSuccess || per_sm < 1) {
-    cudaGetLastError();
-    per_sm = 1;
-  }
-  if (g.tune.sweep_ctas_per_sm > 0) per_sm = std::min(per_sm, g.tune.sweep_ctas_per_sm);
-  return grid_of(B, per_sm);
+// w = L^-1 r, z = L^-T w for every active system.
+int enqueue_sweeps(bsp_batch_s* B, BatchGroup& g, cudaStream_t s) {
+  unsigned* tk = g.tickets.get();
+  BSP_TRY(wave_sweep_multi(B->h, g.lo, g.v_lo, g.R, g.rp.get(), g.w.get(), tk, g.sys_active.get(), s));
+  return wave_sweep_multi(B->h, g.up, g.v_up, g.R, g.w.get(), g.z.get(), tk + 1, g.sys_active.get(), s);
 }
 
-// Enqueues the kernels of one phase of one group; returns the number of kernels.
-int enqueue_group(bsp_batch_s* B, BatchGroup& g, const Kernels& k, cudaStream_t s, bool init) {
+// Enqueues the kernels of one phase of one group and adds their number to n.
+int enqueue_group(bsp_batch_s* B, BatchGroup& g, const Kernels& k, cudaStream_t s, bool init, int& n) {
   const BGroupP v = view(B, g);
   const int tg = grid_of(B, g.tune.ctas_per_sm), tt = g.tune.threads;
   const int fin_grid = (g.n_sys() * 32 + 255) / 256;
-  const BSweepP fw = sweep_params(B, g, true), bw = sweep_params(B, g, false);
-  const int sg_f = sweep_grid(B, g, k.sweep_fwd), sg_b = sweep_grid(B, g, k.sweep_bwd);
   if (init) {
     k.init<<<tg, tt, 0, s>>>(v);
     cudaMemsetAsync(g.sys_active.get(), 1, g.n_sys() * sizeof(int), s);
-    cudaMemsetAsync(g.tickets.get(), 0, 2 * sizeof(unsigned), s);
-    k.sweep_fwd<<<sg_f, kBSweepThreads, 0, s>>>(fw);
-    k.sweep_bwd<<<sg_b, kBSweepThreads, 0, s>>>(bw);
+    BSP_TRY(enqueue_sweeps(B, g, s));
     k.init_dots<<<tg, tt, 0, s>>>(v);
     k.fin_init<<<fin_grid, 256, 0, s>>>(v);
-    return 5;
+    n += 5;
+    return BSP_OK;
   }
   k.spmv<<<tg, tt, 0, s>>>(v);
   k.fin_alpha<<<fin_grid, 256, 0, s>>>(v);
   k.update<<<tg, tt, 0, s>>>(v);
-  k.fin_res<<<fin_grid, 256, 0, s>>>(v);  // also zeroes the sweep tickets
-  k.sweep_fwd<<<sg_f, kBSweepThreads, 0, s>>>(fw);
-  k.sweep_bwd<<<sg_b, kBSweepThreads, 0, s>>>(bw);
+  k.fin_res<<<fin_grid, 256, 0, s>>>(v);
+  BSP_TRY(enqueue_sweeps(B, g, s));
   k.dot_rz<<<tg, tt, 0, s>>>(v);
   k.fin_beta<<<fin_grid, 256, 0, s>>>(v);
   k.pupd<<<tg, tt, 0, s>>>(v);
-  return 9;
+  n += 9;
+  return BSP_OK;
 }
 
 BContP cont_params(bsp_batch_s* B, int max_iters) {
@@ -958,29 +636,86 @@ BContP cont_params(bsp_batch_s* B, int max_iters) {
   return c;
 }
 
-// Fork the phase over the group streams and join back into `s`.
+// Fork the phase over the group streams and join back into `s`; count: kernels.
 int enqueue_phase(bsp_batch_s* B, const std::vector<Kernels>& ks, cudaStream_t s, bool init,
-                  cudaGraphConditionalHandle hnd, int use_cond, int max_iters) {
+                  cudaGraphConditionalHandle hnd, int use_cond, int max_iters, int64_t& count) {
   int n = 0;
   BSP_CUDA_TRY(cudaEventRecord(B->fork, s));
   for (size_t gi = 0; gi < B->groups.size(); ++gi) {
     BSP_CUDA_TRY(cudaStreamWaitEvent(B->gs[gi], B->fork, 0));
-    n += enqueue_group(B, B->groups[gi], ks[gi], B->gs[gi], init);
+    BSP_TRY(enqueue_group(B, B->groups[gi], ks[gi], B->gs[gi], init, n));
     BSP_CUDA_TRY(cudaEventRecord(B->join[gi], B->gs[gi]));
     BSP_CUDA_TRY(cudaStreamWaitEvent(s, B->join[gi], 0));
   }
   k_bt_continue<<<1, 256, 0, s>>>(cont_params(B, max_iters), hnd, use_cond, init ? 0 : 1);
   BSP_CUDA_TRY(cudaPeekAtLastError());
-  return n + 1;
+  count = n + 1;
+  return BSP_OK;
+}
+
+// The factor's sweeps over the group's systems for R right-hand sides: plans,
+// values, and the items of every row.  The preconditioner sorts the lower
+// blocks of a row by column and stores them row by row, the diagonal last.
+int build_sweeps(bsp_batch_s* B, BatchGroup& g, int R) {
+  const int n = (int)g.n_rows();
+  const auto& rp = g.A->h_row_ptr;
+  const auto& ci = g.A->h_col_idx;
+  SweepEntries lo, up;
+  lo.ptr.assign(n + 1, 0);
+  up.ptr.assign(n + 1, 0);
+  std::vector<int> row;
+  int64_t e = 0;
+  for (int i = 0; i < n; ++i) {
+    row.clear();
+    for (int t = rp[i]; t < rp[i + 1]; ++t)
+      if (ci[t] <= i) row.push_back(ci[t]);
+    std::sort(row.begin(), row.end());
+    for (int j : row) {
+      if (j < i) {
+        lo.col.push_back(j);
+        lo.blk.push_back(e);
+        up.ptr[j + 1]++;
+      }
+      ++e;
+    }
+    lo.ptr[i + 1] = (int)lo.col.size();
+  }
+  for (int i = 0; i < n; ++i) up.ptr[i + 1] += up.ptr[i];
+  up.col.resize(lo.col.size());
+  up.blk.resize(lo.col.size());
+  std::vector<int> fill(up.ptr.begin(), up.ptr.end() - 1);
+  for (int i = 0; i < n; ++i)
+    for (int t = lo.ptr[i]; t < lo.ptr[i + 1]; ++t) {
+      const int p = fill[lo.col[t]]++;
+      up.col[p] = i;
+      up.blk[p] = lo.blk[t];
+    }
+  std::vector<int> beg(g.row_off.begin(), g.row_off.end()), il, iu;
+  g.lo = WaveSym{};
+  g.up = WaveSym{};
+  BSP_TRY(wave_build(n, g.bs, false, up, true, true, true, beg, R, nullptr, &iu, g.up));
+  BSP_TRY(wave_build(n, g.bs, true, lo, false, true, false, beg, R, &iu, &il, g.lo));
+  for (auto [d, v] : {std::pair{&g.item_lo, &il}, std::pair{&g.item_up, &iu}}) {
+    BSP_TRY(d->alloc(v->size()));
+    BSP_CUDA_TRY(cudaMemcpy(d->get(), v->data(), v->size() * sizeof(int), cudaMemcpyHostToDevice));
+  }
+  BSP_TRY(wave_gather(B->h, g.lo, BSP_PREC_F64, g.pc->f_vals.get(), g.pc->dinv.get(), g.v_lo));
+  BSP_TRY(wave_gather(B->h, g.up, BSP_PREC_F64, g.pc->f_vals.get(), g.pc->dinv.get(), g.v_up));
+  return BSP_OK;
 }
 
 int alloc_state(bsp_batch_s* B, BatchGroup& g, int R, int hist_cap) {
   if (g.R != R) {
     const size_t nv = (size_t)g.n_rows() * R * g.bs;
-    for (DevBuf<double>* v : {&g.x, &g.r, &g.z, &g.w, &g.p, &g.q}) {
+    if (!g.R || (g.R == 1) != (R == 1)) BSP_TRY(build_sweeps(B, g, R));  // the plans for 2 and 4 are the same
+    for (DevBuf<double>* v : {&g.x, &g.r, &g.z, &g.p, &g.q}) {
       BSP_TRY(v->alloc(nv));
       BSP_CUDA_TRY(cudaMemset(v->get(), 0, nv * sizeof(double)));
     }
+    BSP_TRY(g.rp.alloc(wave_item_values(g.lo, R)));
+    BSP_CUDA_TRY(cudaMemset(g.rp.get(), 0, g.rp.n * sizeof(double)));
+    BSP_TRY(g.w.alloc(wave_item_values(g.up, R)));
+    BSP_CUDA_TRY(cudaMemset(g.w.get(), 0, g.w.n * sizeof(double)));
     BSP_TRY(g.part0.alloc((size_t)g.n_tiles * R));
     BSP_TRY(g.part1.alloc((size_t)g.n_tiles * R));
     BSP_TRY(g.st.alloc((size_t)g.n_sys() * R));
@@ -1019,8 +754,8 @@ float time_ms(cudaStream_t s, const std::function<void()>& f, int reps) {
 }
 
 // Autotuner: time each candidate launch shape on the group's own data.  The
-// candidates compute identical results (reductions are per fixed tile, sweep
-// rows do not depend on scheduling), so only speed differs.
+// candidates compute identical results (reductions are per fixed tile), so only
+// speed differs.
 int autotune(bsp_batch_s* B, BatchGroup& g, const Kernels& k) {
   cudaStream_t s = B->cap;
   BSP_CUDA_TRY(cudaMemsetAsync(g.sys_active.get(), 1, g.n_sys() * sizeof(int), s));
@@ -1045,28 +780,6 @@ int autotune(bsp_batch_s* B, BatchGroup& g, const Kernels& k) {
   }
   g.tune.threads = bestc.threads;
   g.tune.ctas_per_sm = bestc.ctas_per_sm;
-  // sweeps: CTAs per SM of the persistent grid
-  int occ = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k.sweep_fwd, kBSweepThreads, 0);
-  occ = std::max(occ, 1);
-  const BSweepP fw = sweep_params(B, g, true);
-  best = 1e30f;
-  int best_sw = occ;
-  for (int cps : {1, 2, 4, 8}) {
-    if (cps > occ) continue;
-    const int grid = grid_of(B, cps);
-    const float ms = time_ms(s, [&] {
-      k.init<<<grid_of(B, g.tune.ctas_per_sm), g.tune.threads, 0, s>>>(v);
-      cudaMemsetAsync(g.tickets.get(), 0, sizeof(unsigned), s);
-      k.sweep_fwd<<<grid, kBSweepThreads, 0, s>>>(fw);
-    }, 3);
-    bsp::count_launch_add(8);
-    if (ms < best) {
-      best = ms;
-      best_sw = cps;
-    }
-  }
-  g.tune.sweep_ctas_per_sm = best_sw;
   g.tuned = true;
   BSP_CUDA_TRY(cudaStreamSynchronize(s));
   BSP_CUDA_TRY(cudaPeekAtLastError());
@@ -1092,7 +805,7 @@ int build_graphs(bsp_batch_s* B, const std::vector<Kernels>& ks, int mode, int m
     // the loop body runs at least once; from then on its last kernel decides
     BSP_CUDA_TRY(cudaGraphConditionalHandleCreate(&hnd, graph, 1, cudaGraphCondAssignDefault));
     BSP_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
-    B->init_kernels = enqueue_phase(B, ks, s, true, hnd, 0, max_iters);
+    BSP_TRY(enqueue_phase(B, ks, s, true, hnd, 0, max_iters, B->init_kernels));
     BSP_CUDA_TRY(cudaStreamEndCapture(s, &init));
     cudaGraphNode_t init_node, cond_node;
     BSP_CUDA_TRY(cudaGraphAddChildGraphNode(&init_node, graph, nullptr, 0, init));
@@ -1105,7 +818,7 @@ int build_graphs(bsp_batch_s* B, const std::vector<Kernels>& ks, int mode, int m
     BSP_CUDA_TRY(cudaGraphAddNode(&cond_node, graph, &init_node, 1, &cp));
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     BSP_CUDA_TRY(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-    B->body_kernels = enqueue_phase(B, ks, s, false, hnd, 1, max_iters);
+    BSP_TRY(enqueue_phase(B, ks, s, false, hnd, 1, max_iters, B->body_kernels));
     BSP_CUDA_TRY(cudaStreamEndCapture(s, &body));
     const cudaError_t e = cudaGraphInstantiate(&B->exec, graph, 0);
     cudaGraphDestroy(graph);
@@ -1113,10 +826,10 @@ int build_graphs(bsp_batch_s* B, const std::vector<Kernels>& ks, int mode, int m
   } else {
     cudaGraph_t init = nullptr, body = nullptr;
     BSP_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
-    B->init_kernels = enqueue_phase(B, ks, s, true, 0, 0, max_iters);
+    BSP_TRY(enqueue_phase(B, ks, s, true, 0, 0, max_iters, B->init_kernels));
     BSP_CUDA_TRY(cudaStreamEndCapture(s, &init));
     BSP_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
-    B->body_kernels = enqueue_phase(B, ks, s, false, 0, 0, max_iters);
+    BSP_TRY(enqueue_phase(B, ks, s, false, 0, 0, max_iters, B->body_kernels));
     BSP_CUDA_TRY(cudaStreamEndCapture(s, &body));
     cudaError_t e = cudaGraphInstantiate(&B->exec, init, 0);
     if (e == cudaSuccess) e = cudaGraphInstantiate(&B->exec_body, body, 0);
@@ -1217,7 +930,7 @@ int bsp_batch_create(bsp_handle_t h, int n_sys, const int* n_rows, const int* bs
     pp.kind = BSP_PC_ICHOL0;
     pp.precision = BSP_PREC_F64;
     BSP_TRY(bsp_precond_create(h, g.A, &pp, &g.pc));
-    // tiles (never crossing a system) and the system of each sweep task
+    // tiles (never crossing a system)
     std::vector<int> tsys, trow, stile(g.n_sys() + 1, 0);
     for (int i = 0; i < g.n_sys(); ++i) {
       stile[i] = (int)tsys.size();
@@ -1237,16 +950,6 @@ int bsp_batch_create(bsp_handle_t h, int n_sys, const int* n_rows, const int* bs
     BSP_TRY(up(g.tile_row, trow));
     BSP_TRY(up(g.sys_tile, stile));
     BSP_TRY(up(g.sys_row, g.row_off));
-    for (int lower = 1; lower >= 0; --lower) {
-      const int nt = lower ? g.pc->n_task_lo : g.pc->n_task_up;
-      std::vector<int> rows(std::max(nt, 1)), ts(std::max(nt, 1), 0);
-      if (nt)
-        BSP_CUDA_TRY(cudaMemcpy(rows.data(), lower ? g.pc->task_lo_row.get() : g.pc->task_up_row.get(),
-                                nt * sizeof(int), cudaMemcpyDeviceToHost));
-      for (int t = 0; t < nt; ++t)
-        ts[t] = (int)(std::upper_bound(g.row_off.begin(), g.row_off.end(), (int64_t)rows[t]) - g.row_off.begin()) - 1;
-      BSP_TRY(up(lower ? g.task_sys_lo : g.task_sys_up, ts));
-    }
     BSP_TRY(g.sys_active.alloc(g.n_sys()));
     BSP_TRY(g.tickets.alloc(2));
     BSP_CUDA_TRY(cudaMemset(g.tickets.get(), 0, 2 * sizeof(unsigned)));

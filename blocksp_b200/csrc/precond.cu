@@ -1339,7 +1339,7 @@ static int analyse_factor_structure(bsp_precond_s* pc, bool lower_only) {
     if (wave) {
       tri_entries(false);
       pc->wv_up = std::make_shared<WaveSym>();
-      BSP_TRY(wave_build(n, pc->bs, false, ent, false, true, false, {}, nullptr, &up_item, *pc->wv_up));
+      BSP_TRY(wave_build(n, pc->bs, false, ent, false, true, false, {}, 1, nullptr, &up_item, *pc->wv_up));
     }
   } else {
     // L^T backward: row i depends on rows j > i with L_ji present
@@ -1368,7 +1368,7 @@ static int analyse_factor_structure(bsp_precond_s* pc, bool lower_only) {
       ent.col = trow;
       ent.blk = tblk;
       pc->wv_up = std::make_shared<WaveSym>();
-      BSP_TRY(wave_build(n, pc->bs, false, ent, true, true, true, {}, nullptr, &up_item, *pc->wv_up));
+      BSP_TRY(wave_build(n, pc->bs, false, ent, true, true, true, {}, 1, nullptr, &up_item, *pc->wv_up));
     }
     BSP_TRY(upload(pc->t_ptr, tp));
     BSP_TRY(upload(pc->t_row, trow));
@@ -1377,7 +1377,7 @@ static int analyse_factor_structure(bsp_precond_s* pc, bool lower_only) {
   if (wave) {
     tri_entries(true);
     pc->wv_lo = std::make_shared<WaveSym>();
-    BSP_TRY(wave_build(n, pc->bs, true, ent, false, lower_only, false, {}, &up_item, nullptr, *pc->wv_lo));
+    BSP_TRY(wave_build(n, pc->bs, true, ent, false, lower_only, false, {}, 1, &up_item, nullptr, *pc->wv_lo));
   }
   return build_factor_plan(pc, n, ptr, col, diag, lower_only);
 }

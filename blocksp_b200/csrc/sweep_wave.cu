@@ -22,11 +22,11 @@ bool wave_supported(int bs) {
   }
 }
 
-WaveShape wave_shape(int bs) {
+WaveShape wave_shape(int bs, int nrhs) {
   WaveShape s;
   switch (bs) {
 #define BSP_WAVE_CASE(B) \
-  case B: s = wave_shape_of<B>(); break;
+  case B: s = nrhs == 1 ? wave_shape_of<B, 1>() : wave_shape_of<B, 2>(); break;
     BSP_WAVE_SIZES(BSP_WAVE_CASE)
 #undef BSP_WAVE_CASE
     default: break;
@@ -90,7 +90,7 @@ static int gather_t(bsp_handle_s* h, const WaveSym& S, const double* fvals, cons
 static size_t prec_bytes(int prec) { return prec == BSP_PREC_F64 ? 8 : prec == BSP_PREC_F32 ? 4 : 2; }
 size_t wave_val_bytes(const WaveSym& S, int prec) {
   // W items past the last one are read (and dropped)
-  return (size_t)(S.n_blk + (int64_t)wave_shape(S.bs).W * (S.ne + 1)) * S.bs * S.bs * prec_bytes(prec);
+  return (size_t)(S.n_blk + (int64_t)wave_shape(S.bs, 1).W * (S.ne + 1)) * S.bs * S.bs * prec_bytes(prec);
 }
 
 int wave_gather(bsp_handle_s* h, const WaveSym& S, int prec, const double* fvals, const double* dinv, WaveVals& out) {
@@ -124,10 +124,10 @@ template <typename T, typename H> static int upload_as(DevBuf<T>& d, const std::
 }
 
 int wave_build(int n, int bs, bool ascending, const SweepEntries& ent, bool trans_blocks, bool has_d, bool trans_d,
-               const std::vector<int>& group_beg, const std::vector<int>* row_item, std::vector<int>* item_of,
-               WaveSym& S) {
+               const std::vector<int>& group_beg, int nrhs, const std::vector<int>* row_item,
+               std::vector<int>* item_of, WaveSym& S) {
   WavePlan P;
-  if (!wave_plan(n, ascending, wave_shape(bs), has_d, ent, group_beg, P)) {
+  if (!wave_plan(n, ascending, wave_shape(bs, nrhs), has_d, ent, group_beg, P)) {
     record_error("triangular sweep: the dependencies are not triangular, or the stream is too long");
     return BSP_INVALID;
   }
@@ -208,27 +208,20 @@ int wave_prepare(bsp_handle_s* h, const WaveSym& lo, const WaveSym& up, const do
 
 template <int BS, typename VT>
 static int sweep_t(bsp_handle_s* h, const WaveSym& S, const WaveP<VT>& p) {
-  if (S.ne == 2) return S.has_d ? wave_launch<BS, VT, true, 2, 1>(h, p) : wave_launch<BS, VT, false, 2, 1>(h, p);
-  return S.has_d ? wave_launch<BS, VT, true, 3, 1>(h, p) : wave_launch<BS, VT, false, 3, 1>(h, p);
+  count_launch();
+  if (S.ne == 2)
+    return S.has_d ? wave_launch<BS, VT, true, 2, 1>(h, p, h->stream) : wave_launch<BS, VT, false, 2, 1>(h, p, h->stream);
+  return S.has_d ? wave_launch<BS, VT, true, 3, 1>(h, p, h->stream) : wave_launch<BS, VT, false, 3, 1>(h, p, h->stream);
 }
 
 template <typename VT>
 static int sweep_typed(bsp_handle_s* h, const WaveSym& S, const WaveVals& V, const double* rhs, double* x,
                        unsigned* ticket) {
-  WaveP<VT> p{};
-  p.n_super = S.n_super;
-  p.super_step = S.super_step.get();
-  p.super_group = S.super_group.get();
-  p.step = S.step.get();
-  p.rec = S.rec.get();
-  p.ext_row = S.ext_row.get();
-  p.vals = reinterpret_cast<const VT*>(V.vals.get());
+  WaveP<VT> p = wave_params<VT>(h, S, V);
   p.rhs = rhs;
   p.x = x;
   p.xs = S.to_items ? wave_ld_of(S.bs) : S.bs;
-  p.spin_limit = h->spin_limit;
   p.ticket = ticket;
-  p.st = h->ws.status.get();
   switch (S.bs) {
 #define BSP_WAVE_CASE(B) \
   case B: return sweep_t<B, VT>(h, S, p);

@@ -68,10 +68,14 @@ template <int BS> struct WaveDim {
   static constexpr int W = kWaveWarps * IPW / WPI * IPG;
   static constexpr int ECAP = W >= 128 ? 64 : W >= 64 ? 32 : W >= 16 ? 16 : 8;
 };
-template <int BS> inline WaveShape wave_shape_of() {
+// External rows of a step with R right-hand sides: with more than one, what the
+// tile of a 3D grid needs (the fetch warps hold them in registers).
+template <int BS, int R> constexpr int wave_ecap() { return R == 1 ? WaveDim<BS>::ECAP : BS == 4 ? 12 : 8; }
+
+template <int BS, int R> inline WaveShape wave_shape_of() {
   WaveShape s;
   s.W = WaveDim<BS>::W;
-  s.ecap = WaveDim<BS>::ECAP;
+  s.ecap = wave_ecap<BS, R>();
   s.ring = kRing;
   s.slots = kSlots;
   s.item_major = WaveDim<BS>::kItemMajor;
@@ -100,7 +104,8 @@ template <int BS, typename VT, bool HAS_D, int NE, int R> struct WaveCfg {
   static constexpr int DEPTH = kRegs * 2 <= 36 ? 2 : 1;
   static constexpr int LOOK = 2 * DEPTH;  // steps ahead whose headers and records are staged
   static_assert(LOOK + 2 < kSlots, "headers of the steps read ahead are staged");
-  static constexpr int kRows = kRing * M::W + 1 + kSlots * (M::W + M::ECAP);
+  static constexpr int ECAP = wave_ecap<BS, R>();
+  static constexpr int kRows = kRing * M::W + 1 + kSlots * (M::W + ECAP);
   static constexpr int OFF_REC = (kRows * LD * 8 + 15) / 16 * 16;
   static constexpr int OFF_HDR = OFF_REC + kSlots * M::W * 16;  // {first item, items} of every staged step
   static constexpr int OFF_BAR = OFF_HDR + kSlots * 8;
@@ -483,7 +488,7 @@ __global__ void __launch_bounds__(WaveCfg<BS, VT, HAS_D, NE, R>::kThreads, 1) k_
     } else {
       // -------------------------------------------------------------- fetch
       // the rows of a step are named three turns of this warp ahead
-      constexpr int NX = (M::ECAP * RW + 31) / 32;
+      constexpr int NX = (C::ECAP * RW + 31) / 32;
       constexpr int F = kFetchWarps;
       const int* hp = reinterpret_cast<const int*>(p.step + t0) + 1;
       struct Turn {
@@ -537,7 +542,7 @@ __global__ void __launch_bounds__(WaveCfg<BS, VT, HAS_D, NE, R>::kThreads, 1) k_
           }
           if (lane == 0) mbar_wait(empty(slot), phase(t) ^ 1u, true, p.st);
           __syncwarp();
-          double* ex = vec + (size_t)(kRing * W + 1 + kSlots * W + slot * M::ECAP) * LD;
+          double* ex = vec + (size_t)(kRing * W + 1 + kSlots * W + slot * C::ECAP) * LD;
 #pragma unroll
           for (int j = 0; j < NX; ++j)
             if (src[j]) ex[(lane + 32 * j) / RW * LD + (lane + 32 * j) % RW] = v[j];
@@ -569,7 +574,23 @@ __global__ void __launch_bounds__(WaveCfg<BS, VT, HAS_D, NE, R>::kThreads, 1) k_
   }
 }
 
-template <int BS, typename VT, bool HAS_D, int NE, int R> int wave_launch(bsp_handle_s* h, const WaveP<VT>& p) {
+// The arrays of a sweep as the kernel takes them (vectors and ticket aside).
+template <typename VT> WaveP<VT> wave_params(bsp_handle_s* h, const WaveSym& S, const WaveVals& V) {
+  WaveP<VT> p{};
+  p.n_super = S.n_super;
+  p.super_step = S.super_step.get();
+  p.super_group = S.super_group.get();
+  p.step = S.step.get();
+  p.rec = S.rec.get();
+  p.ext_row = S.ext_row.get();
+  p.vals = reinterpret_cast<const VT*>(V.vals.get());
+  p.spin_limit = h->spin_limit;
+  p.st = h->ws.status.get();
+  return p;
+}
+
+template <int BS, typename VT, bool HAS_D, int NE, int R>
+int wave_launch(bsp_handle_s* h, const WaveP<VT>& p, cudaStream_t stream) {
   using C = WaveCfg<BS, VT, HAS_D, NE, R>;
   static bool ready = false;
   auto kern = k_wave<BS, VT, HAS_D, NE, R>;
@@ -578,8 +599,7 @@ template <int BS, typename VT, bool HAS_D, int NE, int R> int wave_launch(bsp_ha
     ready = true;
   }
   const int grid = p.n_super < h->num_sms ? (p.n_super < 1 ? 1 : p.n_super) : h->num_sms;
-  count_launch();
-  kern<<<grid, C::kThreads, C::kSmem, h->stream>>>(p);
+  kern<<<grid, C::kThreads, C::kSmem, stream>>>(p);
   BSP_CUDA_TRY(cudaPeekAtLastError());
   return BSP_OK;
 }

@@ -34,16 +34,17 @@ struct WaveSym {
 
 // Block sizes the lock-step kernel takes (FP64 vectors).
 bool wave_supported(int bs);
-WaveShape wave_shape(int bs);
+WaveShape wave_shape(int bs, int nrhs);
 
 // Plans and uploads the sweep over n rows; ascending: forward (dependencies
-// j < i), else backward (j > i).  group_beg: see wave_plan.  A sweep reads its
+// j < i), else backward (j > i).  group_beg: see wave_plan; nrhs: right-hand
+// sides of a row (the plans for 2 and 4 are the same).  A sweep reads its
 // right-hand side in item order; one that is followed by another writes its
 // result in that one's item order: row_item is, per row, the item that reads
 // it (null: natural order), and item_of receives that of this sweep.
 int wave_build(int n, int bs, bool ascending, const SweepEntries& ent, bool trans_blocks, bool has_d, bool trans_d,
-               const std::vector<int>& group_beg, const std::vector<int>* row_item, std::vector<int>* item_of,
-               WaveSym& S);
+               const std::vector<int>& group_beg, int nrhs, const std::vector<int>* row_item,
+               std::vector<int>* item_of, WaveSym& S);
 // Values of a vector of one value set per item (1 right-hand side).
 size_t wave_item_values(const WaveSym& S, int nrhs);
 
@@ -68,5 +69,11 @@ int wave_prepare(bsp_handle_s* h, const WaveSym& lo, const WaveSym& up, const do
 // the sentinel on entry; the ticket must be 0 and is 0 again afterwards.
 int wave_sweep(bsp_handle_s* h, const WaveSym& S, int prec, const WaveVals& V, const double* rhs, double* x,
                unsigned* ticket);
+
+// The same with nrhs (1, 2 or 4) right-hand sides interleaved per row, FP64, a
+// sweep with D blocks, 4 x 4, 8 x 8 or 16 x 16 blocks, on a stream of its own
+// (it may be capturing).  Rows of a group whose group_active is 0 are skipped.
+int wave_sweep_multi(bsp_handle_s* h, const WaveSym& S, const WaveVals& V, int nrhs, const double* rhs, double* x,
+                     unsigned* ticket, const int* group_active, cudaStream_t stream);
 
 }  // namespace bsp
