@@ -471,7 +471,6 @@ struct BatchGroup {
   // the two sweeps for this R (super-tasks stay inside a system)
   WaveSym lo, up;
   WaveVals v_lo, v_up;
-  DevBuf<int> item_lo, item_up;
   DevBuf<double> x, r, rp, z, w, p, q, part0, part1, hist;
   DevBuf<BState> st;
   DevBuf<int> sys_active;
@@ -542,8 +541,8 @@ BGroupP view(bsp_batch_s* B, BatchGroup& g) {
   v.st = g.st.get();
   v.sys_active = g.sys_active.get();
   v.rp = g.rp.get();
-  v.item_lo = g.item_lo.get();
-  v.item_up = g.item_up.get();
+  v.item_lo = g.lo.item_of.get();
+  v.item_up = g.up.item_of.get();
   v.hist = g.hist_cap > 0 ? g.hist.get() : nullptr;
   v.hist_cap = g.hist_cap;
   v.opts = B->opts.get();
@@ -690,15 +689,11 @@ int build_sweeps(bsp_batch_s* B, BatchGroup& g, int R) {
       up.col[p] = i;
       up.blk[p] = lo.blk[t];
     }
-  std::vector<int> beg(g.row_off.begin(), g.row_off.end()), il, iu;
+  std::vector<int> beg(g.row_off.begin(), g.row_off.end()), iu;
   g.lo = WaveSym{};
   g.up = WaveSym{};
   BSP_TRY(wave_build(n, g.bs, false, up, true, true, true, beg, R, nullptr, &iu, g.up));
-  BSP_TRY(wave_build(n, g.bs, true, lo, false, true, false, beg, R, &iu, &il, g.lo));
-  for (auto [d, v] : {std::pair{&g.item_lo, &il}, std::pair{&g.item_up, &iu}}) {
-    BSP_TRY(d->alloc(v->size()));
-    BSP_CUDA_TRY(cudaMemcpy(d->get(), v->data(), v->size() * sizeof(int), cudaMemcpyHostToDevice));
-  }
+  BSP_TRY(wave_build(n, g.bs, true, lo, false, true, false, beg, R, &iu, nullptr, g.lo));
   BSP_TRY(wave_gather(B->h, g.lo, BSP_PREC_F64, g.pc->f_vals.get(), g.pc->dinv.get(), g.v_lo));
   BSP_TRY(wave_gather(B->h, g.up, BSP_PREC_F64, g.pc->f_vals.get(), g.pc->dinv.get(), g.v_up));
   return BSP_OK;

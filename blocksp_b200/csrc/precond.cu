@@ -1431,6 +1431,24 @@ static int analyse_diag_structure(bsp_precond_s* pc) {
     pc->n_lev_up = level_order(n, false, upper_deps, order);
     BSP_TRY(upload(pc->order_up, order));
     BSP_TRY(make_tasks(pc, false, n, upper_deps));
+    if (wave_supported(pc->bs)) {
+      // the dependent entries of a forward (j < i) and a backward sweep
+      for (const bool fwd : {true, false}) {
+        SweepEntries ent;
+        ent.ptr.assign(n + 1, 0);
+        for (int i = 0; i < n; ++i) {
+          for (int t = rp[i]; t < rp[i + 1]; ++t)
+            if (fwd ? ci[t] < i : ci[t] > i) {
+              ent.col.push_back(ci[t]);
+              ent.blk.push_back(t);
+            }
+          ent.ptr[i + 1] = (int)ent.col.size();
+        }
+        auto& S = fwd ? pc->wv_lo : pc->wv_up;
+        S = std::make_shared<WaveSym>();
+        BSP_TRY(wave_build(n, pc->bs, fwd, ent, false, false, false, {}, 1, nullptr, nullptr, *S));
+      }
+    }
   }
   return BSP_OK;
 }
@@ -1625,6 +1643,35 @@ static int apply_wave(bsp_precond_s* pc, const double* r, double* z) {
   return wave_sweep(h, *pc->wv_up, prec, up, w, z, pc->wticket.get());
 }
 
+// z = M^{-1} r for SOR: nu sweeps each way of x_i = c_i - sum_dep (w D_i A_ij) x_j,
+// c_i formed by a pass over the other entries before each (z may alias r).
+template <typename VT>
+static int apply_sor_wave(bsp_precond_s* pc, const double* r, double* z, const VT* avals, const VT* dinv,
+                          const std::vector<int>& dirs) {
+  bsp_handle_s* h = pc->h;
+  const bsp_matrix_s* A = pc->A;
+  constexpr int prec = prec_of<VT>();
+  const size_t need = std::max(wave_item_values(*pc->wv_lo, 1), wave_item_values(*pc->wv_up, 1));
+  if (pc->s64[2].n < need) BSP_TRY(take(pc->A, pc->s64[2], need));
+  double *rp = pc->s64[2].get(), *bufs[2] = {pc->s64[0].get(), pc->s64[1].get()};
+  const double* xold = nullptr;
+  for (size_t s = 0; s < dirs.size(); ++s) {
+    const bool fwd = dirs[s] < 0;
+    const WaveSym& S = fwd ? *pc->wv_lo : *pc->wv_up;
+    WaveVals& V = fwd ? pc->vv_lo[prec] : pc->vv_up[prec];
+    if (!V.valid) {
+      const size_t vb = wave_val_bytes(S, prec);
+      if (V.vals.n < vb) BSP_TRY(take(pc->A, V.vals, vb));
+      BSP_TRY(wave_gather(h, S, prec, A->vals.get(), pc->dinv.get(), V, true, pc->w));
+    }
+    double* out = s + 1 == dirs.size() ? z : bufs[s & 1];
+    BSP_TRY(wave_sor_prepare(h, S, prec, fwd, A->row_ptr.get(), A->col_idx.get(), avals, dinv, pc->w, r, xold, rp, out));
+    BSP_TRY(wave_sweep(h, S, prec, V, rp, out, pc->wticket.get()));
+    xold = out;
+  }
+  return BSP_OK;
+}
+
 // z = M^{-1} r (z may alias r).  Every sweep with dependencies writes into a
 // buffer pre-filled with the sentinel and reads its right-hand side from a
 // different buffer; sa, sb, sc are scratch vectors of n*bs values.
@@ -1661,16 +1708,19 @@ static int apply_typed(bsp_precond_s* pc, const AT* r, AT* z, const VT* fvals, c
       p.vals = avals;
       p.dinv = dinv;
       p.w = (AT)pc->w;
+      std::vector<int> dirs;
+      if (pc->type < 0) dirs.assign(pc->nu, +1);
+      else if (pc->type == 0) { dirs.assign(pc->nu, -1); dirs.insert(dirs.end(), pc->nu, +1); }
+      else dirs.assign(pc->nu, -1);
+      if constexpr (std::is_same<AT, double>::value) {
+        if (pc->wv_lo && pc->wv_up) return apply_sor_wave<VT>(pc, r, z, avals, dinv, dirs);
+      }
       const AT* rhs = r;
       if (z == r) {  // in place: keep a copy of the right-hand side
         BSP_CUDA_TRY(cudaMemcpyAsync(sc, r, nv * sizeof(AT), cudaMemcpyDeviceToDevice, h->stream));
         rhs = sc;
       }
       p.rhs = rhs;
-      std::vector<int> dirs;
-      if (pc->type < 0) dirs.assign(pc->nu, +1);
-      else if (pc->type == 0) { dirs.assign(pc->nu, -1); dirs.insert(dirs.end(), pc->nu, +1); }
-      else dirs.assign(pc->nu, -1);
       const AT* xold = nullptr;
       AT* bufs[2] = {sa, sb};
       for (size_t s = 0; s < dirs.size(); ++s) {

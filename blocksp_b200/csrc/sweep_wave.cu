@@ -36,11 +36,11 @@ WaveShape wave_shape(int bs, int nrhs) {
 
 // ------------------------------------------------------------------ values
 // Stored block b: minus factor block blk_src[b] (transposed when trans),
-// premultiplied by its row's D when the sweep has D blocks, or what the
+// premultiplied by w times its row's D (PREMUL), or what the
 // negative codes of wave_plan.h say.
-template <int BS, typename VT, bool HAS_D>
+template <int BS, typename VT, bool PREMUL>
 __global__ void k_wave_gather(int64_t nblk, const int64_t* __restrict__ blk_src, const int* __restrict__ blk_row,
-                              const double* __restrict__ src, const double* __restrict__ dinv, int trans, int trans_d,
+                              const double* __restrict__ src, const double* __restrict__ dinv, int trans, int trans_d, double w,
                               VT* __restrict__ dst) {
   constexpr int B2 = BS * BS;
   const int64_t total = nblk * B2;
@@ -52,7 +52,7 @@ __global__ void k_wave_gather(int64_t nblk, const int64_t* __restrict__ blk_src,
     double v = 0.0;
     if (sb >= 0) {
       const double* B = src + sb * B2;
-      if constexpr (HAS_D) {
+      if constexpr (PREMUL) {
         const double* D = dinv + (int64_t)blk_row[b] * B2;
 #pragma unroll
         for (int m = 0; m < BS; ++m)
@@ -60,7 +60,7 @@ __global__ void k_wave_gather(int64_t nblk, const int64_t* __restrict__ blk_src,
       } else {
         v = trans ? B[c * BS + a] : B[a * BS + c];
       }
-      v = -v;
+      v = -w * v;
     } else if (sb == kWaveD) {
       v = dinv[(int64_t)blk_row[b] * B2 + (trans_d ? c * BS + a : a * BS + c)];
     } else if (sb == kWaveOne) {
@@ -73,16 +73,17 @@ __global__ void k_wave_gather(int64_t nblk, const int64_t* __restrict__ blk_src,
 }
 
 template <int BS, typename VT>
-static int gather_t(bsp_handle_s* h, const WaveSym& S, const double* fvals, const double* dinv, WaveVals& out) {
+static int gather_t(bsp_handle_s* h, const WaveSym& S, const double* fvals, const double* dinv, bool premul, double w,
+                    WaveVals& out) {
   const int g = grid_for(h, S.n_blk * BS * BS, 256);
   VT* dst = reinterpret_cast<VT*>(out.vals.get());
   count_launch();
-  if (S.has_d)
+  if (S.has_d || premul)
     k_wave_gather<BS, VT, true><<<g, 256, 0, h->stream>>>(S.n_blk, S.blk_src.get(), S.blk_row.get(), fvals, dinv,
-                                                          S.trans_blocks, S.trans_d, dst);
+                                                          S.trans_blocks, S.trans_d, w, dst);
   else
     k_wave_gather<BS, VT, false><<<g, 256, 0, h->stream>>>(S.n_blk, S.blk_src.get(), S.blk_row.get(), fvals, dinv,
-                                                           S.trans_blocks, S.trans_d, dst);
+                                                           S.trans_blocks, S.trans_d, w, dst);
   BSP_CUDA_TRY(cudaPeekAtLastError());
   return BSP_OK;
 }
@@ -93,7 +94,8 @@ size_t wave_val_bytes(const WaveSym& S, int prec) {
   return (size_t)(S.n_blk + (int64_t)wave_shape(S.bs, 1).W * (S.ne + 1)) * S.bs * S.bs * prec_bytes(prec);
 }
 
-int wave_gather(bsp_handle_s* h, const WaveSym& S, int prec, const double* fvals, const double* dinv, WaveVals& out) {
+int wave_gather(bsp_handle_s* h, const WaveSym& S, int prec, const double* fvals, const double* dinv, WaveVals& out,
+                bool premul, double w) {
   const size_t vb = wave_val_bytes(S, prec);
   if (out.vals.n < vb) BSP_TRY(out.vals.alloc(vb));
   if (S.n_blk > 0) {
@@ -101,9 +103,9 @@ int wave_gather(bsp_handle_s* h, const WaveSym& S, int prec, const double* fvals
     switch (S.bs) {
 #define BSP_WAVE_CASE(B)                                                                      \
   case B:                                                                                     \
-    st = prec == BSP_PREC_F64   ? gather_t<B, double>(h, S, fvals, dinv, out)                 \
-         : prec == BSP_PREC_F32 ? gather_t<B, float>(h, S, fvals, dinv, out)                  \
-                                : gather_t<B, __nv_bfloat16>(h, S, fvals, dinv, out);         \
+    st = prec == BSP_PREC_F64   ? gather_t<B, double>(h, S, fvals, dinv, premul, w, out)                 \
+         : prec == BSP_PREC_F32 ? gather_t<B, float>(h, S, fvals, dinv, premul, w, out)                  \
+                                : gather_t<B, __nv_bfloat16>(h, S, fvals, dinv, premul, w, out);         \
     break;
       BSP_WAVE_SIZES(BSP_WAVE_CASE)
 #undef BSP_WAVE_CASE
@@ -112,6 +114,86 @@ int wave_gather(bsp_handle_s* h, const WaveSym& S, int prec, const double* fvals
     BSP_TRY(st);
   }
   out.valid = true;
+  return BSP_OK;
+}
+
+// ------------------------------------------------------------------ SOR
+// One thread per value of x: the row's product with the old iterate (its
+// threads read a block row each), then the inverted diagonal times the CTA's
+// residuals in shared memory.  A pass over A at most; 40 x 36 x 44 rows of 4 x 4
+// blocks (60 MB, cached in L2): 12 us beside a sweep of 60 us.
+constexpr int kSorThreads = 256;
+template <int BS, typename VT>
+__global__ void __launch_bounds__(kSorThreads)
+k_sor_prepare(int n, int forward, const int* __restrict__ row_ptr, const int* __restrict__ col,
+              const VT* __restrict__ avals, const VT* __restrict__ dinv, double w, const int* __restrict__ item_of,
+              const double* b, const double* __restrict__ xold, double* __restrict__ rp, double* x) {
+  constexpr int RPC = kSorThreads / BS, LD = wave_ld_of(BS);
+  __shared__ double res[RPC][BS];
+  auto val = [](VT v) -> double {
+    if constexpr (sizeof(VT) == 2) return (double)__bfloat162float(v);
+    else return (double)v;
+  };
+  const int lr = threadIdx.x / BS, r = threadIdx.x % BS;
+  const int i = blockIdx.x * RPC + lr;
+  const bool on = lr < RPC && i < n;
+  const int64_t k = (int64_t)i * BS + r;
+  double old = 0.0;
+  if (on) {
+    double t = b[k];
+    if (xold) {
+      old = xold[k];
+      for (int e = __ldg(row_ptr + i); e < __ldg(row_ptr + i + 1); ++e) {
+        const int j = __ldg(col + e);
+        if (forward ? j <= i : j >= i) continue;
+        const VT* a = avals + (int64_t)e * (BS * BS) + r * BS;
+        const double* xj = xold + (int64_t)j * BS;
+        double s = 0.0;
+#pragma unroll
+        for (int c = 0; c < BS; ++c) s = fma(val(a[c]), xj[c], s);
+        t -= s;
+      }
+    }
+    res[lr][r] = t;
+  }
+  __syncthreads();
+  if (on) {
+    const VT* d = dinv + (int64_t)i * (BS * BS) + r * BS;
+    double s = 0.0;
+#pragma unroll
+    for (int c = 0; c < BS; ++c) s = fma(val(d[c]), res[lr][c], s);
+    rp[(int64_t)__ldg(item_of + i) * LD + r] = old + (-w * old + w * s);
+    reinterpret_cast<unsigned long long*>(x)[k] = kSentinel64;
+  }
+}
+
+int wave_sor_prepare(bsp_handle_s* h, const WaveSym& S, int prec, bool forward, const int* row_ptr, const int* col,
+                     const void* avals, const void* dinv, double w, const double* b, const double* xold, double* rp,
+                     double* x) {
+  auto run = [&](auto bs, auto v) -> int {
+    constexpr int BS = decltype(bs)::value;
+    using VT = decltype(v);
+    const int grid = (int)ceil_div(S.n, kSorThreads / BS);
+    count_launch();
+    k_sor_prepare<BS, VT><<<grid, kSorThreads, 0, h->stream>>>(
+        S.n, forward ? 1 : 0, row_ptr, col, static_cast<const VT*>(avals), static_cast<const VT*>(dinv), w,
+        S.item_of.get(), b, xold, rp, x);
+    return BSP_OK;
+  };
+  int st = BSP_INVALID;
+  switch (S.bs) {
+#define BSP_WAVE_CASE(B)                                                               \
+  case B:                                                                              \
+    st = prec == BSP_PREC_F64   ? run(std::integral_constant<int, B>{}, double{})      \
+         : prec == BSP_PREC_F32 ? run(std::integral_constant<int, B>{}, float{})       \
+                                : run(std::integral_constant<int, B>{}, __nv_bfloat16{}); \
+    break;
+    BSP_WAVE_SIZES(BSP_WAVE_CASE)
+#undef BSP_WAVE_CASE
+    default: break;
+  }
+  BSP_TRY(st);
+  BSP_CUDA_TRY(cudaPeekAtLastError());
   return BSP_OK;
 }
 
@@ -131,11 +213,10 @@ int wave_build(int n, int bs, bool ascending, const SweepEntries& ent, bool tran
     record_error("triangular sweep: the dependencies are not triangular, or the stream is too long");
     return BSP_INVALID;
   }
-  if (item_of) {
-    item_of->assign(n, 0);
-    for (size_t i = 0; i < P.item_row.size(); ++i)
-      if (P.item_row[i] >= 0) (*item_of)[P.item_row[i]] = (int)i;
-  }
+  std::vector<int> items(n, 0);
+  for (size_t i = 0; i < P.item_row.size(); ++i)
+    if (P.item_row[i] >= 0) items[P.item_row[i]] = (int)i;
+  BSP_TRY(upload_as(S.item_of, items));
   if (row_item) {
     for (auto& r : P.rec)
       if (r.row >= 0) r.row = (*row_item)[r.row];
@@ -160,6 +241,7 @@ int wave_build(int n, int bs, bool ascending, const SweepEntries& ent, bool tran
   BSP_TRY(upload_as(S.ext_row, P.ext_row));
   BSP_TRY(upload_as(S.blk_src, P.blk_src));
   BSP_TRY(upload_as(S.blk_row, P.blk_row));
+  if (item_of) *item_of = std::move(items);
   return BSP_OK;
 }
 

@@ -27,6 +27,7 @@ struct WaveSym {
   bool to_items = false;  // its result goes to the item order of the sweep that follows
   bool trans_blocks = false, has_d = false, trans_d = false;
   DevBuf<int> super_step, super_group, item_row, ext_row, blk_row;
+  DevBuf<int> item_of;  // per row: the item that reads its right-hand side
   DevBuf<int2> step;
   DevBuf<int4> rec;
   DevBuf<int64_t> blk_src;
@@ -57,13 +58,24 @@ size_t wave_val_bytes(const WaveSym& S, int prec);
 
 // Gathers the stream's values (into a buffer of at least wave_val_bytes) from
 // the factor (FP64, factor entry order) and the D blocks from dinv (FP64, row
-// order), converted to the precision `prec` (BSP_PREC_F64 / F32 / BF16).
-int wave_gather(bsp_handle_s* h, const WaveSym& S, int prec, const double* fvals, const double* dinv, WaveVals& out);
+// order), converted to the precision `prec` (BSP_PREC_F64 / F32 / BF16).  premul:
+// the blocks of a sweep without D blocks are w D_r B_e all the same.
+int wave_gather(bsp_handle_s* h, const WaveSym& S, int prec, const double* fvals, const double* dinv, WaveVals& out,
+                bool premul = false, double w = 1.0);
 
 // Start of z = M^-1 r through the sweeps lo, then up (z may alias r): rp = r in
 // lo's item order, w (up's item order) and z filled with the sentinel.
 int wave_prepare(bsp_handle_s* h, const WaveSym& lo, const WaveSym& up, const double* r, double* rp, double* w,
                  double* z);
+
+// Start of one SOR sweep (blocksp_preconditioners.hpp:116-240): the part of
+//   x_i = (1 - w) xold_i + w D_i (b_i - sum_j A_ij x_j)
+// that does not depend on the sweep, in S's item order (the sums over rows that
+// the sweep visits later, from xold; null: 0), and x filled with the sentinel (x
+// may be b).  A's rows in the precision of the solve, D = inverted diagonals.
+int wave_sor_prepare(bsp_handle_s* h, const WaveSym& S, int prec, bool forward, const int* row_ptr, const int* col,
+                     const void* avals, const void* dinv, double w, const double* b, const double* xold, double* rp,
+                     double* x);
 
 // x = sweep(rhs) on h's stream, one right-hand side, FP64 vectors.  x must hold
 // the sentinel on entry; the ticket must be 0 and is 0 again afterwards.

@@ -65,6 +65,21 @@ def test_long_rows_and_far_rows(handle, bs, n, w, wide):
     check(handle, band_system(n, bs, w, 5, wide))
 
 
+@pytest.mark.parametrize("bs", [1, 2, 3, 4, 5, 6, 8, 16])
+@pytest.mark.parametrize("kind,nu", [(0, 3), (1, 1), (1, 2), (-1, 1), (-1, 2)])
+def test_sor(handle, bs, kind, nu):
+    """SOR on the same sweeps: one and several, each way and both (in place)."""
+    import blocksp_b200 as bsp
+    for s in (grid_system((37, 33), bs, seed=6), grid_system((5, 6, 7), bs, seed=6, skew=0.3),
+              band_system(60, bs, 9, 2), grid_system((1, 1), bs, seed=6)):
+        A, Ao = bsp.Matrix.from_system(s, handle), O.BSR.from_system(s)
+        r = np.random.default_rng(8).uniform(-1, 1, s.n * bs)
+        pc = bsp.SOR(A, 1.3, nu, kind)
+        assert rel(pc.apply_host(r), O.SOR(Ao, 1.3, nu, kind)(r.copy())) <= 1e-11
+        pc.close()
+        A.close()
+
+
 @pytest.mark.parametrize("bs", [4, 8])
 def test_vectors_aligned_to_one_value(handle, torch_cuda, bs):
     import blocksp_b200 as bsp
