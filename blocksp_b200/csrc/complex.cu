@@ -17,8 +17,8 @@
 // So pGMRES and its deflated restart are restated here in complex arithmetic
 // (blocksp_solvers.hpp:107-295, blocksp_deflated_restart.hpp:38-269, complex
 // branches): dot(x, y) = sum conj(x_i) y_i (blocksp_utility.hpp:277-292), the
-// Arnoldi step on the device (complex dot and axpy kernels over the
-// interleaved vectors), the small dense work (least squares, harmonic Ritz
+// Arnoldi step on the device (one launch of complex modified Gram-Schmidt,
+// mgs.cuh, over the interleaved vectors), the small dense work (least squares, harmonic Ritz
 // values, complex Schur form and its reordering) on the host.  The reference
 // has no complex pCG / IChol0 (static_asserts at blocksp_solvers.hpp:55, 411,
 // 485); neither has this library.
@@ -29,6 +29,7 @@
 #include <limits>
 #include <vector>
 #include "complex_dense.h"
+#include "mgs.cuh"
 #include "reduce.cuh"
 #include "precond.hpp"
 
@@ -66,6 +67,10 @@ struct Store2Fin {
     out[0] = s[0];
     out[1] = s[1];
   }
+};
+struct NormOfFin {
+  double* out;
+  __device__ void operator()(const double (&s)[1]) const { *out = sqrt(fabs(s[0])); }
 };
 // Reduction body: sum |y_c|^2 = dot(y, y).
 struct CNormBody {
@@ -165,6 +170,14 @@ int pgmres_complex_solve(bsp_handle_s* h, bsp_matrix_s* A, bsp_precond_s* pc, co
   BSP_TRY(h->scratch("cgmres.r0", len, &r0));
   BSP_TRY(h->scratch("cgmres.scalars", (size_t)2 * (cols + 2), &dsc));
   std::vector<double> hsc((size_t)2 * (cols + 2));
+  double **qtab = nullptr, *mgs_part = nullptr, *thresh = nullptr;
+  unsigned* mgs_bar = nullptr;
+  BSP_TRY(h->scratch("cgmres.qtab", cols + 1, &qtab));
+  BSP_TRY(h->scratch("cgmres.mgs_partials", (size_t)2 * kMgsSums * h->num_sms, &mgs_part));
+  BSP_TRY(h->scratch("cgmres.mgs_barrier", 1, &mgs_bar));
+  BSP_TRY(h->scratch("cgmres.thresh", 1, &thresh));
+  int n_tab = 0;    // basis vectors named in qtab
+  int written = 1;  // basis vectors formed so far
   const int g = grid_for(h, nc, 256);
   cudaStream_t st = h->stream;
   EventTimer tm(st);
@@ -188,6 +201,7 @@ int pgmres_complex_solve(bsp_handle_s* h, bsp_matrix_s* A, bsp_precond_s* pc, co
   BSP_CUDA_TRY(cudaMemsetAsync(x0, 0, len * sizeof(double), st));
   const double zero_thresh = std::min(res_mag.back() * kEpsC, kEpsC);
   const double tolerance = res_mag.back() * o->tol;
+  BSP_CUDA_TRY(cudaMemcpyAsync(thresh, &zero_thresh, sizeof(double), cudaMemcpyHostToDevice, st));
   int iter = 0, tot = 0, n_restarts = 0;
   CMat H(1, 0);
   std::vector<Cx> y, c_r;
@@ -202,24 +216,37 @@ int pgmres_complex_solve(bsp_handle_s* h, bsp_matrix_s* A, bsp_precond_s* pc, co
     H = Hg;
     BSP_TRY(bsmv_launch(A, 1, 0, BSP_F64, 1.0, Q[iter], 0.0, nullptr, w, st));
     if (pc) BSP_TRY(precond_apply(pc, BSP_PREC_F64, w, w));
-    for (int j = 0; j <= iter; ++j) {
-      BSP_TRY(launch_reduce<2>(h, 0, nc, CDotBody{reinterpret_cast<const double2*>(Q[j]),
-                                                  reinterpret_cast<const double2*>(w)},
-                               Store2Fin{dsc + 2 * j}));
-      bsp::count_launch(), k_caxpy_dev<<<g, 256, 0, st>>>(nc, dsc + 2 * j, reinterpret_cast<const double2*>(Q[j]),
-                                                          reinterpret_cast<double2*>(w));
+    // the basis grows by a few vectors at a time where memory allows
+    if ((int)Q.size() < iter + 2)
+      for (int i = (int)Q.size(); i < std::min(iter + 8, cols) && basis(i); ++i) {}
+    if (!basis(iter + 1)) return BSP_OUT_OF_MEMORY;
+    if ((int)Q.size() > n_tab) {  // its table on the device
+      n_tab = (int)Q.size();
+      BSP_CUDA_TRY(cudaMemcpyAsync(qtab, Q.data(), n_tab * sizeof(double*), cudaMemcpyHostToDevice, st));
     }
-    BSP_TRY(launch_reduce<1>(h, 0, nc, CNormBody{reinterpret_cast<const double2*>(w)},
-                             StoreFin{dsc + 2 * (iter + 1)}));
+    // one launch when w's slices fit, else a dot and an axpy per basis vector
+    const int mg = launch_mgs<true>(h, len, w, qtab, iter, dsc, 2, thresh, mgs_part, mgs_bar);
+    if (mg > 1) return mg;
+    if (mg == 1) {
+      for (int j = 0; j <= iter; ++j) {
+        BSP_TRY(launch_reduce<2>(h, 0, nc, CDotBody{reinterpret_cast<const double2*>(Q[j]),
+                                                    reinterpret_cast<const double2*>(w)},
+                                 Store2Fin{dsc + 2 * j}));
+        bsp::count_launch(), k_caxpy_dev<<<g, 256, 0, st>>>(nc, dsc + 2 * j, reinterpret_cast<const double2*>(Q[j]),
+                                                            reinterpret_cast<double2*>(w));
+      }
+      BSP_TRY(launch_reduce<1>(h, 0, nc, CNormBody{reinterpret_cast<const double2*>(w)},
+                               NormOfFin{dsc + 2 * (iter + 1)}));
+    }
     BSP_CUDA_TRY(cudaMemcpyAsync(hsc.data(), dsc, (size_t)(2 * (iter + 1) + 1) * sizeof(double),
                                  cudaMemcpyDeviceToHost, st));
     BSP_CUDA_TRY(cudaStreamSynchronize(st));
     for (int j = 0; j <= iter; ++j) H(j, iter) = Cx(hsc[2 * j], hsc[2 * j + 1]);
-    const double hn = std::sqrt(std::fabs(hsc[2 * (iter + 1)]));
+    const double hn = hsc[2 * (iter + 1)];
     if (!std::isfinite(hn)) return BSP_NAN;
     H(iter + 1, iter) = hn;
-    if (!(hn < zero_thresh)) {
-      if (!basis(iter + 1)) return BSP_OUT_OF_MEMORY;
+    if (!(hn < zero_thresh)) written = std::max(written, iter + 2);
+    if (mg == 1 && !(hn < zero_thresh)) {
       bsp::count_launch(), k_cdiv<<<grid_for(h, len, 256), 256, 0, st>>>(len, hn, w, Q[iter + 1]);
     }
     // residual: min || c - H y || (c = ||r_0|| e_1, or c_r after a restart)
@@ -259,7 +286,7 @@ int pgmres_complex_solve(bsp_handle_s* h, bsp_matrix_s* A, bsp_precond_s* pc, co
         iter = 0;
         restarted = false;
       } else {
-        if ((int)Q.size() < H.r) return BSP_BREAKDOWN;  // the last Arnoldi step broke down
+        if (written < H.r) return BSP_BREAKDOWN;  // the last Arnoldi step broke down
         CMat Pk1, Hnew;
         if (deflate_complex(H, res_vec, k, Pk1, Hnew, c_r) != 0) {
           record_error("deflated restart: the complex Schur iteration did not converge");
