@@ -297,14 +297,48 @@ __global__ void k_gm_init(GPtrs g, double tol) {
   if (!isfinite(res0)) h->done = DONE_NAN;
 }
 
-// Least-squares update after column j was built (H(0..j+1, j) in place).
-__global__ void k_gm_ls(GPtrs g, int max_iters) {
+// Least-squares update after column j was built (H(0..j+1, j) in place).  One
+// warp: the column and the rotations are brought to shared memory (one thread
+// working in global memory took 20 us a column at restart 30, mostly load
+// latency; this takes 5), where lane 0 applies sd::ls_add_column's operations
+// in the same order.  Columns longer than the stage stay in global memory.
+constexpr int kLsRows = 1024, kLsRots = 128;
+__global__ void __launch_bounds__(32) k_gm_ls(GPtrs g, int max_iters) {
+  __shared__ double col[kLsRows];
+  __shared__ sd::Rot rot[kLsRots];
   KHead* h = g.head;
+  const int lane = threadIdx.x;
   const int j = h->j;
   const double hsub = g.H[(j + 1) * g.m + j];
-  if (fabs(hsub) < h->zero_thresh) h->breakdown = 1;
   int nrot = *g.nrot;
-  const double res = sd::ls_add_column(g.H, g.m, j, j + 1, g.R, g.rots, nrot, g.g);
+  double res = 0.0;
+  if (j + 2 <= kLsRows) {
+    for (int i = lane; i <= j + 1; i += 32) col[i] = g.H[i * g.m + j];
+    for (int t0 = 0; t0 < nrot; t0 += kLsRots) {
+      const int n = min(kLsRots, nrot - t0);
+      __syncwarp();
+      for (int t = lane; t < n; t += 32) rot[t] = g.rots[t0 + t];
+      __syncwarp();
+      if (lane == 0)
+        for (int t = 0; t < n; ++t) sd::apply_rot(rot[t], col, 1);
+    }
+    if (lane == 0) {
+      sd::Rot q;
+      q.p = j;
+      sd::make_givens(col[j], col[j + 1], q.c, q.s);
+      sd::apply_rot(q, col, 1);
+      col[j + 1] = 0.0;
+      sd::apply_rot(q, g.g, 1);
+      g.rots[nrot++] = q;
+      res = sd::dabs(g.g[j + 1]);
+    }
+    __syncwarp();
+    for (int i = lane; i <= j + 1; i += 32) g.R[i * g.m + j] = col[i];
+  } else if (lane == 0) {
+    res = sd::ls_add_column(g.H, g.m, j, j + 1, g.R, g.rots, nrot, g.g);
+  }
+  if (lane != 0) return;
+  if (fabs(hsub) < h->zero_thresh) h->breakdown = 1;
   *g.nrot = nrot;
   h->res = res;
   if (h->n_hist < g.hist_cap) g.hist[h->n_hist] = res;
@@ -857,7 +891,7 @@ int pgmres_solve(bsp_handle_s* h, bsp_matrix_s* A, bsp_precond_s* pc, const doub
                                NormFin{gp.H + (size_t)(j + 1) * m + j}));
       bsp::count_launch(), k_div<<<g, 256, 0, h->stream>>>(len, vv.get(), gp.H + (size_t)(j + 1) * m + j, hd, qptr[j + 1]);
     }
-    bsp::count_launch(), k_gm_ls<<<1, 1, 0, h->stream>>>(gp, o->max_iters);
+    bsp::count_launch(), k_gm_ls<<<1, 32, 0, h->stream>>>(gp, o->max_iters);
     BSP_CUDA_TRY(cudaPeekAtLastError());
     BSP_TRY(read_head(h, hd, &st));
     if (st.done != DONE_RUNNING) break;
