@@ -327,6 +327,9 @@ int bsp_handle_destroy(bsp_handle_t h) {
     DeviceGuard g(h->device);
     cudaStreamSynchronize(h->stream);
     h->ws = Workspace{};
+    if (h->pin) cudaFreeHost(h->pin);
+    for (auto e : h->pin_event)
+      if (e) cudaEventDestroy(e);
     if (h->own_stream) cudaStreamDestroy(h->stream);
   }
   delete h;

@@ -166,6 +166,20 @@ struct bsp_handle_s {
     *out = reinterpret_cast<T*>(b.p);
     return 0;
   }
+  // pinned slots for small state words on their way to the host, with an event each
+  static constexpr int kPinnedSlots = 4;
+  static constexpr size_t kPinnedSlot = 256;
+  unsigned char* pin = nullptr;
+  cudaEvent_t pin_event[kPinnedSlots] = {};
+  int pinned() {
+    if (pin) return 0;
+    for (auto& e : pin_event)
+      if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return BSP_CUDA_ERROR;
+    void* q = nullptr;
+    if (cudaMallocHost(&q, kPinnedSlots * kPinnedSlot) != cudaSuccess) return BSP_OUT_OF_MEMORY;
+    pin = static_cast<unsigned char*>(q);
+    return 0;
+  }
   int stage(size_t n_in, size_t n_out) {
     if (stage_in.n < n_in) { int s = stage_in.alloc(n_in); if (s) return s; }
     if (stage_out.n < n_out) { int s = stage_out.alloc(n_out); if (s) return s; }

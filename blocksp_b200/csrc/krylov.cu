@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstring>
 #include <type_traits>
 #include <vector>
 #include "reduce.cuh"
@@ -150,9 +151,12 @@ struct CgPApBody {
     for (int k = 0; k < kC; ++k) a[0] = fma(pv.v[k], av.v[k], a[0]);
   }
 };
+// The host runs an iteration ahead of what it has read: once the solve has
+// ended (head->done) the kernels below change nothing that it returns.
 struct CgPApFin {
   KHead* head;
   __device__ void operator()(const double (&s)[1]) const {
+    if (head->done != DONE_RUNNING) return;
     head->pAp = s[0];
     head->alpha = head->rz / s[0];  // alpha = rz / dot(p, Ap)
   }
@@ -163,8 +167,13 @@ struct CgUpdBody {  // x += alpha p; r -= alpha Ap; sum r.r
   const KHead* head;
   double alpha;
   int64_t n;
-  __device__ void setup() { alpha = head->alpha; }
+  bool run;
+  __device__ void setup() {
+    alpha = head->alpha;
+    run = head->done == DONE_RUNNING;
+  }
   __device__ void operator()(int64_t c, double (&a)[1]) {
+    if (!run) return;
     const int64_t e = c * kC;
     V4 xv = ld4(x, e, n), rv = ld4(r, e, n);
     const V4 pv = ld4(p, e, n), av = ld4(Ap, e, n);
@@ -183,6 +192,7 @@ struct CgUpdFin {
   double* hist;
   int hist_cap;
   __device__ void operator()(const double (&s)[1]) const {
+    if (head->done != DONE_RUNNING) return;
     const double res = sqrt(s[0]);
     head->res = res;
     if (head->n_hist < hist_cap) hist[head->n_hist] = res;
@@ -205,6 +215,7 @@ struct CgRzFin {
   KHead* head;
   int max_iters;
   __device__ void operator()(const double (&s)[1]) const {
+    if (head->done != DONE_RUNNING) return;
     head->beta = s[0] / head->rz;  // beta = dot(r, z) / rz
     head->rz = s[0];
     head->j++;
@@ -302,11 +313,13 @@ __global__ void k_gm_init(GPtrs g, double tol) {
 // working in global memory took 20 us a column at restart 30, mostly load
 // latency; this takes 5), where lane 0 applies sd::ls_add_column's operations
 // in the same order.  Columns longer than the stage stay in global memory.
+// A solve that has ended is left as it is (the host runs a step ahead).
 constexpr int kLsRows = 1024, kLsRots = 128;
 __global__ void __launch_bounds__(32) k_gm_ls(GPtrs g, int max_iters) {
   __shared__ double col[kLsRows];
   __shared__ sd::Rot rot[kLsRots];
   KHead* h = g.head;
+  if (h->done != DONE_RUNNING) return;
   const int lane = threadIdx.x;
   const int j = h->j;
   const double hsub = g.H[(j + 1) * g.m + j];
@@ -659,6 +672,40 @@ static int read_head(bsp_handle_s* h, const KHead* d, KHead* out) {
   return BSP_OK;
 }
 
+// Copies of the state word on their way to the host, one per step.
+struct HeadReader {
+  bsp_handle_s* h;
+  const KHead* head;
+  static constexpr int kSlots = 4;
+  static_assert(sizeof(KHead) <= bsp_handle_s::kPinnedSlot, "a state word per pinned slot");
+  HeadReader(bsp_handle_s* hh, const KHead* d) : h(hh), head(d) {}
+  int post(int i) {
+    BSP_TRY(h->pinned());
+    const int s = i % kSlots;
+    BSP_CUDA_TRY(cudaMemcpyAsync(h->pin + s * bsp_handle_s::kPinnedSlot, head, sizeof(KHead), cudaMemcpyDeviceToHost,
+                                 h->stream));
+    BSP_CUDA_TRY(cudaEventRecord(h->pin_event[s], h->stream));
+    return BSP_OK;
+  }
+  int read(int i, KHead* out) {
+    const int s = i % kSlots;
+    BSP_CUDA_TRY(cudaEventSynchronize(h->pin_event[s]));
+    memcpy(out, h->pin + s * bsp_handle_s::kPinnedSlot, sizeof(KHead));
+    return BSP_OK;
+  }
+  // Whether the step on its way is unlikely to be the solve's last one, so that
+  // the next is worth queueing before its state is read: the residual would
+  // have to fall by more than the square of its last reduction.  A wrong guess
+  // costs time only (a step that changes nothing, or a gap).
+  double before = 0.0, last = 0.0;
+  bool ahead(const KHead& st) {
+    if (st.res != last) before = last, last = st.res;
+    if (!(before > 0.0)) return true;
+    const double f = std::min(last / before, 1.0);
+    return last * f * f > st.tolerance;
+  }
+};
+
 static int status_of(int done) {
   switch (done) {
     case DONE_CONVERGED: return BSP_OK;
@@ -717,19 +764,30 @@ int pcg_solve(bsp_handle_s* h, bsp_matrix_s* A, bsp_precond_s* pc, const double*
   BSP_TRY(launch_reduce<2>(h, 3, chunks_of(len), CgInitBody{vp.get(), vr.get(), len}, CgInitFin{hd, o->tol, dhist.get()}));
   KHead st;
   BSP_TRY(read_head(h, hd, &st));
-  while (st.done == DONE_RUNNING) {
+  // An iteration is queued behind the one whose state is read, so the device
+  // does not wait for the host (24 x 20 rows of 2 x 2 blocks: 100 us an
+  // iteration with two synchronising reads, 83 us so).  One that runs after
+  // the solve has ended changes nothing.
+  HeadReader heads(h, hd);
+  auto iteration = [&](int i) -> int {
     BSP_TRY(bsmv_launch(A, 1, 0, op_dtype, 1.0,vp.get(), 0.0, nullptr, vAp.get(), h->stream));
     BSP_TRY(launch_reduce<1>(h, 4, chunks_of(len), CgPApBody{vp.get(), vAp.get(), len}, CgPApFin{hd}));
-    BSP_TRY(launch_reduce<1>(h, 5, chunks_of(len), CgUpdBody{x, vr.get(), vp.get(), vAp.get(), hd, 0.0, len},
+    BSP_TRY(launch_reduce<1>(h, 5, chunks_of(len), CgUpdBody{x, vr.get(), vp.get(), vAp.get(), hd, 0.0, len, true},
                              CgUpdFin{hd, dhist.get(), hcap}));
-    BSP_TRY(read_head(h, hd, &st));
-    if (st.done != DONE_RUNNING) break;
     if (pc) BSP_TRY(precond_apply(pc, op_prec,vr.get(), vz.get()));
     else bsp::count_launch(), k_copy<<<g, 256, 0, h->stream>>>(len, vr.get(), vz.get());
     BSP_TRY(launch_reduce<1>(h, 6, chunks_of(len), CgRzBody{vr.get(), vz.get(), len}, CgRzFin{hd, o->max_iters}));
     bsp::count_launch(), k_cg_p<<<g, 256, 0, h->stream>>>(len, vz.get(), hd, vp.get());
     BSP_CUDA_TRY(cudaPeekAtLastError());
-    BSP_TRY(read_head(h, hd, &st));
+    return heads.post(i);
+  };
+  if (st.done == DONE_RUNNING) {
+    int queued = 0;
+    for (int i = 0; st.done == DONE_RUNNING; ++i) {
+      const int upto = i < o->max_iters && heads.ahead(st) ? i + 1 : i;
+      for (; queued <= upto; ++queued) BSP_TRY(iteration(queued));
+      BSP_TRY(heads.read(i, &st));
+    }
   }
   const double solve_ms = tm.stop_ms();
   if (pc) BSP_TRY(precond_check_status(pc));
@@ -870,11 +928,10 @@ int pgmres_solve(bsp_handle_s* h, bsp_matrix_s* A, bsp_precond_s* pc, const doub
   KHead st;
   BSP_TRY(read_head(h, hd, &st));
   int n_restarts = 0;
-  // first Arnoldi steps reuse the zeroed memset of q_0 normalisation guard
-  while (st.done == DONE_RUNNING) {
-    const int j = st.j;
+  HeadReader heads(h, hd);
+  // column j: v = M^-1 A q_j, Gram-Schmidt, least squares
+  auto column = [&](int j) -> int {
     BSP_TRY(ensure_basis(j + 2));
-    // v = M^-1 A q_j
     BSP_TRY(bsmv_launch(A, 1, 0, op_dtype, 1.0,qptr[j], 0.0, nullptr, vv.get(), h->stream));
     if (pc) BSP_TRY(precond_apply(pc, op_prec,vv.get(), vv.get()));
     // MGS: one persistent launch when v's slices fit, else j+2 fused passes
@@ -893,7 +950,22 @@ int pgmres_solve(bsp_handle_s* h, bsp_matrix_s* A, bsp_precond_s* pc, const doub
     }
     bsp::count_launch(), k_gm_ls<<<1, 32, 0, h->stream>>>(gp, o->max_iters);
     BSP_CUDA_TRY(cudaPeekAtLastError());
-    BSP_TRY(read_head(h, hd, &st));
+    return heads.post(j);
+  };
+  bool queued = false;  // column st.j is on its way already
+  while (st.done == DONE_RUNNING) {
+    const int j = st.j;
+    if (!queued) BSP_TRY(column(j));
+    // the next column is queued before this one's state is read, except where
+    // a restart or the end of the solve comes first or no room is left for it
+    // (a column past the end of the solve is not used)
+    queued = j + 1 < m && st.tot < o->max_iters && heads.ahead(st);
+    if (queued && ensure_basis(j + 3) != BSP_OK) {
+      cudaGetLastError();
+      queued = false;
+    }
+    if (queued) BSP_TRY(column(j + 1));
+    BSP_TRY(heads.read(j, &st));
     if (st.done != DONE_RUNNING) break;
     if (restart > 0 && st.j == restart) {
       // x_0 = x_0 + Q y
