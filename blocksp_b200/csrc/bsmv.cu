@@ -10,9 +10,13 @@
 // warp reads 512 contiguous bytes, the blocks are read exactly once with
 // evict-first caching, and x (which is re-read ~7 times for a 7-point stencil)
 // stays resident in the 126 MB L2.  The CPR lanes that share a block row are
-// reduced with shuffles.  This is an HBM-bound kernel: arithmetic intensity is
+// reduced with shuffles.  ld values lie between the block rows of x, z and y:
+// BS * R where all right-hand sides go through in one launch (FULL, kept a
+// constant: 90^3 rows of 4 x 4 blocks with 2 right-hand sides take 154 us so
+// and 176 with ld at run time).  This is an HBM-bound kernel: arithmetic intensity is
 // 2 flop per stored value (R right-hand sides: 2R), far below any tensor-core
 // ridge point, so it runs on the FP64/FP32 pipes.
+#include "bsmv_rows.hpp"
 #include "internal.hpp"
 
 namespace bsp {
@@ -20,9 +24,9 @@ namespace bsp {
 constexpr int kBsmvThreads = 256;
 constexpr int kUnroll = 4;
 
-template <int BS, typename VT, typename AT, int R>
+template <int BS, typename VT, typename AT, int R, bool FULL>
 __global__ void __launch_bounds__(kBsmvThreads)
-k_bsmv(int n_rows, const int* __restrict__ row_ptr, const int* __restrict__ col_idx,
+k_bsmv(int n_rows, int64_t ld_, const int* __restrict__ row_ptr, const int* __restrict__ col_idx,
        const VT* __restrict__ vals, const AT* __restrict__ x, AT alpha, AT beta,
        const AT* z, AT* y) {
   using M = BlockMap<BS, VT>;
@@ -32,6 +36,7 @@ k_bsmv(int n_rows, const int* __restrict__ row_ptr, const int* __restrict__ col_
   const int row = blockIdx.x * (kBsmvThreads / G) + threadIdx.x / G;
   const bool valid = row < n_rows;
   const int c0 = (gl % CPR) * V;
+  const int64_t ld = FULL ? (int64_t)(BS * R) : ld_;
   const CV* vblk = reinterpret_cast<const CV*>(vals);
 
   AT acc[P][R];
@@ -58,7 +63,7 @@ k_bsmv(int n_rows, const int* __restrict__ row_ptr, const int* __restrict__ col_
 #pragma unroll
         for (int r = 0; r < R; ++r) {
           AT xv[V];
-          ld_vec<V>(x + (int64_t)cols[u] * (BS * R) + r * BS + c0, xv);
+          ld_vec<V>(x + (int64_t)cols[u] * ld + r * BS + c0, xv);
 #pragma unroll
           for (int p = 0; p < P; ++p) {
             AT av[V];
@@ -77,7 +82,7 @@ k_bsmv(int n_rows, const int* __restrict__ row_ptr, const int* __restrict__ col_
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         AT xv[V];
-        ld_vec<V>(x + (int64_t)col * (BS * R) + r * BS + c0, xv);
+        ld_vec<V>(x + (int64_t)col * ld + r * BS + c0, xv);
 #pragma unroll
         for (int p = 0; p < P; ++p) {
           AT av[V];
@@ -98,7 +103,7 @@ k_bsmv(int n_rows, const int* __restrict__ row_ptr, const int* __restrict__ col_
     for (int p = 0; p < P; ++p)
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        const int64_t yi = (int64_t)row * (BS * R) + r * BS + p * RPP + gl / CPR;
+        const int64_t yi = (int64_t)row * ld + r * BS + p * RPP + gl / CPR;
         AT out = alpha * acc[p][r];
         if (beta != AT(0)) out += beta * z[yi];
         y[yi] = out;
@@ -112,7 +117,7 @@ k_bsmv(int n_rows, const int* __restrict__ row_ptr, const int* __restrict__ col_
 // contributes A[r][c0+v] * x_i[r] to y_j[c0+v]).
 template <int BS, typename VT, typename AT, int R>
 __global__ void __launch_bounds__(kBsmvThreads)
-k_bsmv_tr(int n_cols, const int* __restrict__ tr_ptr, const int* __restrict__ tr_row,
+k_bsmv_tr(int n_cols, int64_t ld, const int* __restrict__ tr_ptr, const int* __restrict__ tr_row,
           const int64_t* __restrict__ tr_blk, const VT* __restrict__ vals,
           const AT* __restrict__ x, AT alpha, AT beta, const AT* z, AT* y) {
   using M = BlockMap<BS, VT>;
@@ -140,7 +145,7 @@ k_bsmv_tr(int n_cols, const int* __restrict__ tr_ptr, const int* __restrict__ tr
         const int rib = p * RPP + gl / CPR;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-          const AT xr = __ldg(x + (int64_t)i * (BS * R) + r * BS + rib);
+          const AT xr = __ldg(x + (int64_t)i * ld + r * BS + rib);
 #pragma unroll
           for (int v = 0; v < V; ++v) acc[r][v] = fma(av[v], xr, acc[r][v]);
         }
@@ -159,7 +164,7 @@ k_bsmv_tr(int n_cols, const int* __restrict__ tr_ptr, const int* __restrict__ tr
     for (int r = 0; r < R; ++r)
 #pragma unroll
       for (int v = 0; v < V; ++v) {
-        const int64_t yi = (int64_t)colb * (BS * R) + r * BS + c0 + v;
+        const int64_t yi = (int64_t)colb * ld + r * BS + c0 + v;
         AT out = alpha * acc[r][v];
         if (beta != AT(0)) out += beta * z[yi];
         y[yi] = out;
@@ -167,120 +172,70 @@ k_bsmv_tr(int n_cols, const int* __restrict__ tr_ptr, const int* __restrict__ tr
   }
 }
 
-// Fallback for any block size / rhs count: one thread per output scalar.
-template <typename VT, typename AT>
-__global__ void k_bsmv_generic(int n_rows, int bs, int R, const int* __restrict__ row_ptr,
-                               const int* __restrict__ col_idx, const VT* __restrict__ vals,
-                               const AT* __restrict__ x, AT alpha, AT beta, const AT* z, AT* y) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t per_row = (int64_t)bs * R;
-  if (idx >= (int64_t)n_rows * per_row) return;
-  const int row = (int)(idx / per_row);
-  const int rem = (int)(idx % per_row);
-  const int r = rem / bs, t = rem % bs;
-  AT acc = AT(0);
-  for (int j = row_ptr[row]; j < row_ptr[row + 1]; ++j) {
-    const int col = col_idx[j];
-    const VT* a = vals + (int64_t)j * bs * bs + (int64_t)t * bs;
-    const AT* xv = x + (int64_t)col * per_row + (int64_t)r * bs;
-    for (int c = 0; c < bs; ++c) acc = fma(AT(a[c]), xv[c], acc);
-  }
-  AT out = alpha * acc;
-  if (beta != AT(0)) out += beta * z[idx];
-  y[idx] = out;
-}
-
-template <typename VT, typename AT>
-__global__ void k_bsmv_tr_generic(int n_cols, int bs, int R, const int* __restrict__ tr_ptr,
-                                  const int* __restrict__ tr_row, const int64_t* __restrict__ tr_blk,
-                                  const VT* __restrict__ vals, const AT* __restrict__ x, AT alpha,
-                                  AT beta, const AT* z, AT* y) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t per_row = (int64_t)bs * R;
-  if (idx >= (int64_t)n_cols * per_row) return;
-  const int colb = (int)(idx / per_row);
-  const int rem = (int)(idx % per_row);
-  const int r = rem / bs, c = rem % bs;
-  AT acc = AT(0);
-  for (int t = tr_ptr[colb]; t < tr_ptr[colb + 1]; ++t) {
-    const int i = tr_row[t];
-    const VT* a = vals + tr_blk[t] * bs * bs;
-    const AT* xv = x + (int64_t)i * per_row + (int64_t)r * bs;
-    for (int rr = 0; rr < bs; ++rr) acc = fma(AT(a[(int64_t)rr * bs + c]), xv[rr], acc);
-  }
-  AT out = alpha * acc;
-  if (beta != AT(0)) out += beta * z[idx];
-  y[idx] = out;
-}
-
 // ------------------------------------------------------------------------
-template <int BS, typename VT, typename AT, int R>
-static void launch_fwd(const bsp_matrix_s* A, const VT* vals, const AT* x, AT alpha, AT beta,
-                       const AT* z, AT* y, cudaStream_t s) {
-  constexpr int G = BlockMap<BS, VT>::G;
-  const int rows_per_cta = kBsmvThreads / G;
-  const int grid = (int)ceil_div(A->n_rows, rows_per_cta);
-  bsp::count_launch(), k_bsmv<BS, VT, AT, R><<<grid, kBsmvThreads, 0, s>>>(A->n_rows, A->row_ptr.get(),
-                                                      A->col_idx.get(), vals, x, alpha, beta, z, y);
-}
-template <int BS, typename VT, typename AT, int R>
-static void launch_tr(const bsp_matrix_s* A, const VT* vals, const AT* x, AT alpha, AT beta,
-                      const AT* z, AT* y, cudaStream_t s) {
-  constexpr int G = BlockMap<BS, VT>::G;
-  const int per_cta = kBsmvThreads / G;
-  const int grid = (int)ceil_div(A->n_cols, per_cta);
-  bsp::count_launch(), k_bsmv_tr<BS, VT, AT, R><<<grid, kBsmvThreads, 0, s>>>(
-      A->n_cols, A->tr_ptr.get(), A->tr_row.get(), A->tr_blk.get(), vals, x, alpha, beta, z, y);
+template <int BS, typename VT, typename AT, int R, bool FULL>
+static void launch_chunked(const bsp_matrix_s* A, int64_t ld, bool tr, const VT* vals, const AT* x, AT alpha, AT beta,
+                           const AT* z, AT* y, cudaStream_t s) {
+  constexpr int per_cta = kBsmvThreads / BlockMap<BS, VT>::G;
+  const int grid = (int)ceil_div(tr ? A->n_cols : A->n_rows, per_cta);
+  if (tr)
+    bsp::count_launch(), k_bsmv_tr<BS, VT, AT, R><<<grid, kBsmvThreads, 0, s>>>(
+        A->n_cols, ld, A->tr_ptr.get(), A->tr_row.get(), A->tr_blk.get(), vals, x, alpha, beta, z, y);
+  else
+    bsp::count_launch(), k_bsmv<BS, VT, AT, R, FULL><<<grid, kBsmvThreads, 0, s>>>(
+        A->n_rows, ld, A->row_ptr.get(), A->col_idx.get(), vals, x, alpha, beta, z, y);
 }
 
-template <int BS, typename VT, typename AT>
-static bool dispatch_r(const bsp_matrix_s* A, int R, bool tr, const VT* vals, const AT* x,
-                       AT alpha, AT beta, const AT* z, AT* y, cudaStream_t s) {
-  if constexpr (BS % Chunk<VT>::V != 0) {
+// R of the right-hand sides held ld apart; false where the size has no kernel.
+template <typename VT, typename AT, int R>
+static bool dispatch_chunked(const bsp_matrix_s* A, int64_t ld, bool tr, const VT* vals, const AT* x, AT alpha, AT beta,
+                             const AT* z, AT* y, cudaStream_t s) {
+  switch (A->bs) {
+#define BSP_BS_CASE(BB)                                                                     \
+  case BB:                                                                                  \
+    if constexpr (BB % Chunk<VT>::V == 0) {                                                 \
+      if (ld == BB * R)                                                                     \
+        launch_chunked<BB, VT, AT, R, true>(A, ld, tr, vals, x, alpha, beta, z, y, s);      \
+      else                                                                                  \
+        launch_chunked<BB, VT, AT, R, false>(A, ld, tr, vals, x, alpha, beta, z, y, s);     \
+      return true;                                                                          \
+    }                                                                                       \
     return false;
-  } else {
-    switch (R) {
-#define BSP_R_CASE(RR)                                                  \
-  case RR:                                                              \
-    if (tr) launch_tr<BS, VT, AT, RR>(A, vals, x, alpha, beta, z, y, s); \
-    else launch_fwd<BS, VT, AT, RR>(A, vals, x, alpha, beta, z, y, s);   \
-    return true;
-      BSP_R_CASE(1)
-      BSP_R_CASE(2)
-      BSP_R_CASE(3)
-      BSP_R_CASE(4)
-#undef BSP_R_CASE
-      default:
-        return false;
-    }
+    BSP_BS_CASE(2)
+    BSP_BS_CASE(4)
+    BSP_BS_CASE(8)
+    BSP_BS_CASE(16)
+    BSP_BS_CASE(32)
+#undef BSP_BS_CASE
+    default:
+      return false;
   }
 }
 
+// The right-hand sides go through the kernels in groups of at most four, as
+// even as they come (5 = 3 + 2): the matrix is read once a group, where a
+// thread per output value read it once a right-hand side (56^3 rows of 8 x 8
+// blocks, 5 right-hand sides: 507 us to 338; 20^3 of 32 x 32: 1045 to 183).  16-byte chunks
+// need a power-of-two block size that holds whole ones and vectors on 16-byte
+// boundaries; the rest takes one thread per scalar row.
 template <typename VT, typename AT>
 static int bsmv_typed(const bsp_matrix_s* A, int R, bool tr, const VT* vals, const AT* x,
                       AT alpha, AT beta, const AT* z, AT* y, cudaStream_t s) {
-  bool done = false;
-  switch (A->bs) {
-    case 2: done = dispatch_r<2, VT, AT>(A, R, tr, vals, x, alpha, beta, z, y, s); break;
-    case 4: done = dispatch_r<4, VT, AT>(A, R, tr, vals, x, alpha, beta, z, y, s); break;
-    case 8: done = dispatch_r<8, VT, AT>(A, R, tr, vals, x, alpha, beta, z, y, s); break;
-    case 16: done = dispatch_r<16, VT, AT>(A, R, tr, vals, x, alpha, beta, z, y, s); break;
-    case 32: done = dispatch_r<32, VT, AT>(A, R, tr, vals, x, alpha, beta, z, y, s); break;
-    default: break;
-  }
-  if (!done) {
-    const int64_t total = (int64_t)(tr ? A->n_cols : A->n_rows) * A->bs * R;
-    const int threads = 256;
-    const int64_t grid = ceil_div(total, threads);
-    if (grid > 0) {
-      if (tr)
-        bsp::count_launch(), k_bsmv_tr_generic<VT, AT><<<(unsigned)grid, threads, 0, s>>>(
-            A->n_cols, A->bs, R, A->tr_ptr.get(), A->tr_row.get(), A->tr_blk.get(), vals, x,
-            alpha, beta, z, y);
-      else
-        bsp::count_launch(), k_bsmv_generic<VT, AT><<<(unsigned)grid, threads, 0, s>>>(
-            A->n_rows, A->bs, R, A->row_ptr.get(), A->col_idx.get(), vals, x, alpha, beta, z, y);
-    }
+  const int64_t ld = (int64_t)A->bs * R;
+  const bool aligned = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  for (int r0 = 0, groups = (R + 3) / 4; groups > 0; --groups) {
+    const int n = (R - r0 + groups - 1) / groups;
+    const int64_t o = (int64_t)r0 * A->bs;
+    const AT* zo = z ? z + o : z;
+    bool done = false;
+    if (aligned) switch (n) {
+        case 1: done = dispatch_chunked<VT, AT, 1>(A, ld, tr, vals, x + o, alpha, beta, zo, y + o, s); break;
+        case 2: done = dispatch_chunked<VT, AT, 2>(A, ld, tr, vals, x + o, alpha, beta, zo, y + o, s); break;
+        case 3: done = dispatch_chunked<VT, AT, 3>(A, ld, tr, vals, x + o, alpha, beta, zo, y + o, s); break;
+        default: done = dispatch_chunked<VT, AT, 4>(A, ld, tr, vals, x + o, alpha, beta, zo, y + o, s); break;
+      }
+    if (!done) bsmv_rows(A, n, ld, tr, vals, x + o, alpha, beta, zo, y + o, s);
+    r0 += n;
   }
   BSP_CUDA_TRY(cudaPeekAtLastError());
   return BSP_OK;
