@@ -18,9 +18,9 @@
 //     the super-tasks of every system in one launch, a system's own plan each;
 //   * right-hand sides are interleaved per block row (the solArray<T,bs,R>
 //     layout), so each matrix / factor block is read once for all R of them;
-//   * per-pair scalars come from segmented reductions over fixed 64-row tiles
-//     that never cross a system: one warp per tile, then one warp per system
-//     sums its tiles in tile order, so results do not depend on launch shape;
+//   * per-pair scalars come from segmented reductions over fixed tiles of a few
+//     rows that never cross a system: one warp per tile, then one CTA per system
+//     sums its tiles in a fixed order, so results do not depend on launch shape;
 //   * one pCG iteration of every group (groups run on forked streams) is
 //     captured as a CUDA graph; the loop is a device-side `while` conditional
 //     node whose condition the last kernel of each iteration sets, so the whole
@@ -42,7 +42,13 @@
 
 namespace bsp {
 
-constexpr int kTileRows = 64;
+// Rows of a tile, the work of one warp: four passes of as many rows as a warp
+// takes at once in the product.  The kernels over tiles are bound by the loads
+// that one warp waits for pass after pass, so a tile is short and the group has
+// tens of thousands: with 64 rows to a tile 25 k rows of 8 x 8 blocks ran on
+// 400 warps (four right-hand sides: product 240 us, update 82, search direction
+// 43; now 54, 22 and 12).
+constexpr int tile_rows(int bs) { return bs == 4 ? 16 : 4; }
 constexpr int kBatchMaxThreads = 512;
 constexpr int kBatchMaxGroups = 4;
 enum { BT_RUNNING = 0, BT_CONVERGED = 1, BT_MAXIT = 2, BT_NAN = 4 };
@@ -105,7 +111,7 @@ __global__ void __launch_bounds__(kBatchMaxThreads) k_bt_spmv(const BGroupP g) {
     const int s = __ldg(g.tile_sys + t);
     if (!g.sys_active[s]) continue;
     const int r0 = __ldg(g.tile_row + t);
-    const int r1 = (int)min((int64_t)r0 + kTileRows, g.sys_row[s + 1]);
+    const int r1 = (int)min((int64_t)r0 + tile_rows(BS), g.sys_row[s + 1]);
     double dot[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) dot[r] = 0.0;
@@ -224,7 +230,7 @@ __global__ void __launch_bounds__(kBatchMaxThreads) k_bt_update(const BGroupP g)
     const int s = __ldg(g.tile_sys + t);
     if (!g.sys_active[s]) continue;
     const int r0 = __ldg(g.tile_row + t);
-    const int r1 = (int)min((int64_t)r0 + kTileRows, g.sys_row[s + 1]);
+    const int r1 = (int)min((int64_t)r0 + tile_rows(BS), g.sys_row[s + 1]);
     bool run[R];
     double al[R], acc[R];
     load_pair_state<R>(g, s, run, al, true);
@@ -258,7 +264,7 @@ __global__ void __launch_bounds__(kBatchMaxThreads) k_bt_dot_rz(const BGroupP g)
     const int s = __ldg(g.tile_sys + t);
     if (!g.sys_active[s]) continue;
     const int r0 = __ldg(g.tile_row + t);
-    const int r1 = (int)min((int64_t)r0 + kTileRows, g.sys_row[s + 1]);
+    const int r1 = (int)min((int64_t)r0 + tile_rows(BS), g.sys_row[s + 1]);
     double acc[R];
 #pragma unroll
     for (int k = 0; k < R; ++k) acc[k] = 0.0;
@@ -278,7 +284,7 @@ __global__ void __launch_bounds__(kBatchMaxThreads) k_bt_pupd(const BGroupP g) {
     const int s = __ldg(g.tile_sys + t);
     if (!g.sys_active[s]) continue;
     const int r0 = __ldg(g.tile_row + t);
-    const int r1 = (int)min((int64_t)r0 + kTileRows, g.sys_row[s + 1]);
+    const int r1 = (int)min((int64_t)r0 + tile_rows(BS), g.sys_row[s + 1]);
     bool run[R];
     double be[R];
     load_pair_state<R>(g, s, run, be, false);
@@ -298,7 +304,7 @@ __global__ void __launch_bounds__(kBatchMaxThreads) k_bt_init(const BGroupP g) {
   BT_FOR_TILES(g, t) {
     const int s = __ldg(g.tile_sys + t);
     const int r0 = __ldg(g.tile_row + t);
-    const int r1 = (int)min((int64_t)r0 + kTileRows, g.sys_row[s + 1]);
+    const int r1 = (int)min((int64_t)r0 + tile_rows(BS), g.sys_row[s + 1]);
     BT_FOR_ELEMS(e, rhs, r0, r1) {
       (void)rhs;
       g.x[e] = 0.0;
@@ -315,7 +321,7 @@ __global__ void __launch_bounds__(kBatchMaxThreads) k_bt_init_dots(const BGroupP
   BT_FOR_TILES(g, t) {
     const int s = __ldg(g.tile_sys + t);
     const int r0 = __ldg(g.tile_row + t);
-    const int r1 = (int)min((int64_t)r0 + kTileRows, g.sys_row[s + 1]);
+    const int r1 = (int)min((int64_t)r0 + tile_rows(BS), g.sys_row[s + 1]);
     double a[R], b[R];
 #pragma unroll
     for (int k = 0; k < R; ++k) a[k] = b[k] = 0.0;
@@ -337,20 +343,21 @@ __global__ void __launch_bounds__(kBatchMaxThreads) k_bt_init_dots(const BGroupP
 // ------------------------------------------------------------------ per-pair scalars
 enum { FIN_INIT = 0, FIN_ALPHA = 1, FIN_RES = 2, FIN_BETA = 3 };
 
-// One warp per system: sums the system's tile partials in tile order, then
+// One CTA per system: sums the system's tile partials in a fixed order, then
 // updates the state of each of its R pairs (solvers.hpp:57-97).
+constexpr int kFinThreads = 256;
 template <int R, int MODE>
-__global__ void k_bt_fin(const BGroupP g) {
-  const int s = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (s >= g.n_sys) return;
+__global__ void __launch_bounds__(kFinThreads) k_bt_fin(const BGroupP g) {
+  __shared__ double part[2][kFinThreads / 32][R];
+  const int s = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (MODE != FIN_INIT && !g.sys_active[s]) return;
   const int t0 = g.sys_tile[s], t1 = g.sys_tile[s + 1];
   const double* src = (MODE == FIN_RES) ? g.part1 : g.part0;
   double a[R], b[R];
 #pragma unroll
   for (int k = 0; k < R; ++k) a[k] = b[k] = 0.0;
-  for (int t = t0 + lane; t < t1; t += 32) {
+#pragma unroll 4
+  for (int t = t0 + (int)threadIdx.x; t < t1; t += kFinThreads) {
 #pragma unroll
     for (int k = 0; k < R; ++k) {
       a[k] += src[(int64_t)t * R + k];
@@ -361,8 +368,19 @@ __global__ void k_bt_fin(const BGroupP g) {
   for (int k = 0; k < R; ++k) {
     a[k] = warp_sum(a[k]);
     if (MODE == FIN_INIT) b[k] = warp_sum(b[k]);
+    if (lane == 0) part[0][warp][k] = a[k], part[1][warp][k] = b[k];
   }
-  if (lane != 0) return;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    a[k] = b[k] = 0.0;
+#pragma unroll
+    for (int w = 0; w < kFinThreads / 32; ++w) {
+      a[k] += part[0][w][k];
+      b[k] += part[1][w][k];
+    }
+  }
   const double tol = g.opts->tol;
   const int max_iters = g.opts->max_iters;
   int any = 0;
@@ -599,23 +617,23 @@ int enqueue_sweeps(bsp_batch_s* B, BatchGroup& g, cudaStream_t s) {
 int enqueue_group(bsp_batch_s* B, BatchGroup& g, const Kernels& k, cudaStream_t s, bool init, int& n) {
   const BGroupP v = view(B, g);
   const int tg = grid_of(B, g.tune.ctas_per_sm), tt = g.tune.threads;
-  const int fin_grid = (g.n_sys() * 32 + 255) / 256;
+  const int fin_grid = g.n_sys();
   if (init) {
     k.init<<<tg, tt, 0, s>>>(v);
     cudaMemsetAsync(g.sys_active.get(), 1, g.n_sys() * sizeof(int), s);
     BSP_TRY(enqueue_sweeps(B, g, s));
     k.init_dots<<<tg, tt, 0, s>>>(v);
-    k.fin_init<<<fin_grid, 256, 0, s>>>(v);
+    k.fin_init<<<fin_grid, kFinThreads, 0, s>>>(v);
     n += 5;
     return BSP_OK;
   }
   k.spmv<<<tg, tt, 0, s>>>(v);
-  k.fin_alpha<<<fin_grid, 256, 0, s>>>(v);
+  k.fin_alpha<<<fin_grid, kFinThreads, 0, s>>>(v);
   k.update<<<tg, tt, 0, s>>>(v);
-  k.fin_res<<<fin_grid, 256, 0, s>>>(v);
+  k.fin_res<<<fin_grid, kFinThreads, 0, s>>>(v);
   BSP_TRY(enqueue_sweeps(B, g, s));
   k.dot_rz<<<tg, tt, 0, s>>>(v);
-  k.fin_beta<<<fin_grid, 256, 0, s>>>(v);
+  k.fin_beta<<<fin_grid, kFinThreads, 0, s>>>(v);
   k.pupd<<<tg, tt, 0, s>>>(v);
   n += 9;
   return BSP_OK;
@@ -929,7 +947,7 @@ int bsp_batch_create(bsp_handle_t h, int n_sys, const int* n_rows, const int* bs
     std::vector<int> tsys, trow, stile(g.n_sys() + 1, 0);
     for (int i = 0; i < g.n_sys(); ++i) {
       stile[i] = (int)tsys.size();
-      for (int64_t r = g.row_off[i]; r < g.row_off[i + 1]; r += kTileRows) {
+      for (int64_t r = g.row_off[i]; r < g.row_off[i + 1]; r += tile_rows(g.bs)) {
         tsys.push_back(i);
         trow.push_back((int)r);
       }
