@@ -35,13 +35,16 @@ WaveShape wave_shape(int bs, int nrhs) {
 }
 
 // ------------------------------------------------------------------ values
-// Stored block b: minus factor block blk_src[b] (transposed when trans),
-// premultiplied by w times its row's D (PREMUL), or what the
-// negative codes of wave_plan.h say.
-template <int BS, typename VT, bool PREMUL>
-__global__ void k_wave_gather(int64_t nblk, const int64_t* __restrict__ blk_src, const int* __restrict__ blk_row,
-                              const double* __restrict__ src, const double* __restrict__ dinv, int trans, int trans_d, double w,
-                              VT* __restrict__ dst) {
+// Stored block b: minus w times factor block blk_src[b] (transposed when
+// trans), or what the negative codes of wave_plan.h say.
+template <typename VT> __device__ __forceinline__ void store_as(VT* p, double v) {
+  if constexpr (sizeof(VT) == 8) *p = v;
+  else if constexpr (sizeof(VT) == 4) *p = (float)v;
+  else *p = __float2bfloat16_rn((float)v);
+}
+template <int BS, typename VT>
+__global__ void k_wave_gather(int64_t nblk, const int64_t* __restrict__ blk_src, const double* __restrict__ src,
+                              int trans, double w, VT* __restrict__ dst) {
   constexpr int B2 = BS * BS;
   const int64_t total = nblk * B2;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
@@ -50,40 +53,87 @@ __global__ void k_wave_gather(int64_t nblk, const int64_t* __restrict__ blk_src,
     const int a = WaveDim<BS>::kChunk ? k / BS : k % BS, c = WaveDim<BS>::kChunk ? k % BS : k / BS;
     const int64_t sb = blk_src[b];
     double v = 0.0;
-    if (sb >= 0) {
-      const double* B = src + sb * B2;
-      if constexpr (PREMUL) {
-        const double* D = dinv + (int64_t)blk_row[b] * B2;
+    if (sb >= 0) v = -w * (trans ? src[sb * B2 + c * BS + a] : src[sb * B2 + a * BS + c]);
+    else if (sb == kWaveOne) v = a == c ? 1.0 : 0.0;
+    store_as(dst + t, v);
+  }
+}
+
+// The same with the block premultiplied by its row's D.  Every value takes BS
+// products, so a CTA brings UB groups of NB blocks and their D to shared memory
+// first (rows one value further apart than they are long: both orders are read
+// without conflicts), each block read from memory once and in order: 484 us
+// for the backward sweep of the 64^3 grid of 8 x 8 blocks, 424 for 44 x 40 x 36
+// of 16 x 16 kept in FP32 (a thread a value that read D and the block itself
+// took 555 and 986).
+constexpr int kGatherThreads = 256;
+template <int BS, typename VT>
+__global__ void __launch_bounds__(kGatherThreads)
+k_wave_gather_d(int64_t nblk, const int64_t* __restrict__ blk_src, const int* __restrict__ blk_row,
+                const double* __restrict__ src, const double* __restrict__ dinv, int trans, int trans_d, double w,
+                VT* __restrict__ dst) {
+  constexpr int B2 = BS * BS, NB = kGatherThreads / B2, UB = 4, LD = BS + 1;
+  static_assert(NB >= 1, "a block per group of threads");
+  __shared__ double sB[UB][NB][BS * LD], sD[UB][NB][BS * LD];
+  const int nb = threadIdx.x / B2, k = threadIdx.x % B2;
+  const int kr = k / BS, kc = k % BS;  // this thread's value of the blocks it loads
+  const int a = WaveDim<BS>::kChunk ? kr : kc, c = WaveDim<BS>::kChunk ? kc : kr;  // and of those it stores
+  const int da = trans_d ? 1 : LD, dm = trans_d ? LD : 1, bm = trans ? 1 : LD, bc = trans ? LD : 1;
+  for (int64_t b0 = (int64_t)blockIdx.x * (UB * NB); b0 < nblk; b0 += (int64_t)gridDim.x * (UB * NB)) {
+    int64_t sb[UB];
+    double vb[UB], vd[UB];
 #pragma unroll
-        for (int m = 0; m < BS; ++m)
-          v = fma(trans_d ? D[m * BS + a] : D[a * BS + m], trans ? B[c * BS + m] : B[m * BS + c], v);
-      } else {
-        v = trans ? B[c * BS + a] : B[a * BS + c];
+    for (int u = 0; u < UB; ++u) {
+      const int64_t b = b0 + u * NB + nb;
+      sb[u] = kWaveZero;
+      vb[u] = vd[u] = 0.0;
+      if (nb < NB && b < nblk) {
+        sb[u] = __ldg(blk_src + b);
+        if (sb[u] >= 0) vb[u] = __ldcs(src + sb[u] * B2 + k);
+        if (sb[u] >= 0 || sb[u] == kWaveD) vd[u] = __ldg(dinv + (int64_t)__ldg(blk_row + b) * B2 + k);
       }
-      v = -w * v;
-    } else if (sb == kWaveD) {
-      v = dinv[(int64_t)blk_row[b] * B2 + (trans_d ? c * BS + a : a * BS + c)];
-    } else if (sb == kWaveOne) {
-      v = a == c ? 1.0 : 0.0;
     }
-    if constexpr (sizeof(VT) == 8) dst[t] = v;
-    else if constexpr (sizeof(VT) == 4) dst[t] = (float)v;
-    else dst[t] = __float2bfloat16_rn((float)v);
+    if (nb < NB)
+#pragma unroll
+      for (int u = 0; u < UB; ++u) {
+        sB[u][nb][kr * LD + kc] = vb[u];
+        sD[u][nb][kr * LD + kc] = vd[u];
+      }
+    __syncthreads();
+    if (nb < NB)
+#pragma unroll
+      for (int u = 0; u < UB; ++u) {
+        const int64_t b = b0 + u * NB + nb;
+        if (b >= nblk) continue;
+        double v = 0.0;
+        if (sb[u] >= 0) {
+#pragma unroll
+          for (int m = 0; m < BS; ++m) v = fma(sD[u][nb][a * da + m * dm], sB[u][nb][m * bm + c * bc], v);
+          v = -w * v;
+        } else if (sb[u] == kWaveD) {
+          v = sD[u][nb][a * da + c * dm];
+        } else if (sb[u] == kWaveOne) {
+          v = a == c ? 1.0 : 0.0;
+        }
+        store_as(dst + b * B2 + k, v);
+      }
+    __syncthreads();
   }
 }
 
 template <int BS, typename VT>
 static int gather_t(bsp_handle_s* h, const WaveSym& S, const double* fvals, const double* dinv, bool premul, double w,
                     WaveVals& out) {
-  const int g = grid_for(h, S.n_blk * BS * BS, 256);
   VT* dst = reinterpret_cast<VT*>(out.vals.get());
   count_launch();
-  if (S.has_d || premul)
-    k_wave_gather<BS, VT, true><<<g, 256, 0, h->stream>>>(S.n_blk, S.blk_src.get(), S.blk_row.get(), fvals, dinv,
-                                                          S.trans_blocks, S.trans_d, w, dst);
-  else
-    k_wave_gather<BS, VT, false><<<g, 256, 0, h->stream>>>(S.n_blk, S.blk_src.get(), S.blk_row.get(), fvals, dinv,
-                                                           S.trans_blocks, S.trans_d, w, dst);
+  if (S.has_d || premul) {
+    const int g = grid_for(h, ceil_div(S.n_blk, 4 * (kGatherThreads / (BS * BS))) * kGatherThreads, kGatherThreads);
+    k_wave_gather_d<BS, VT><<<g, kGatherThreads, 0, h->stream>>>(S.n_blk, S.blk_src.get(), S.blk_row.get(), fvals, dinv,
+                                                                 S.trans_blocks, S.trans_d, w, dst);
+  } else {
+    const int g = grid_for(h, S.n_blk * BS * BS, 256);
+    k_wave_gather<BS, VT><<<g, 256, 0, h->stream>>>(S.n_blk, S.blk_src.get(), fvals, S.trans_blocks, w, dst);
+  }
   BSP_CUDA_TRY(cudaPeekAtLastError());
   return BSP_OK;
 }
