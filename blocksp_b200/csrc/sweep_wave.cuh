@@ -32,12 +32,12 @@
 // once.  One application (two sweeps and the preparation), measured against
 // the kernels this replaced (level-ordered polling rows; for 8 x 8 and 16 x 16
 // blocks chains that polled shared memory):
-//   ILU0   64^3, 8 x 8           377 -> 322 us (2.99 TB/s)
-//   ILU0   48^3, 16 x 16         720 -> 358 us
-//   IChol0 300 x 257, 4 x 4     4825 -> 388 us (556 levels, twice)
-//   ILU0   40 x 36 x 44, 4 x 4   718 -> 137 us
-//   IChol0 64 x 64, 4 x 4        704 ->  89 us
-//   IChol0 24 x 20, 2 x 2        273 ->  43 us
+//   ILU0   64^3, 8 x 8           377 -> 300 us (3.2 TB/s)
+//   ILU0   48^3, 16 x 16         720 -> 351 us
+//   IChol0 300 x 257, 4 x 4     4825 -> 360 us (556 levels, twice)
+//   ILU0   40 x 36 x 44, 4 x 4   718 -> 125 us
+//   IChol0 64 x 64, 4 x 4        704 ->  85 us
+//   IChol0 24 x 20, 2 x 2        273 ->  39 us
 // A polling hop cost 4.6 us a level there; here only rows that cross a CTA are
 // polled (about 1.3 us each).  Tried and worse: blocks staged in shared memory
 // by bulk copies and read back (twice the shared-memory traffic, 0.7 us a
@@ -50,22 +50,28 @@
 
 namespace bsp {
 
-constexpr int kFetchWarps = 2;
 constexpr int kWaveWarps = 8;   // compute warps of a set
 constexpr int kSlots = 8;       // steps staged ahead
 constexpr int kRing = 8;        // steps whose results stay in shared memory
 
 // Lanes and CTA shape of a block size.  Sizes 1, 2, 4, 8, 16: row-major
-// blocks, lane l of a block holds pieces q * 32 + l of V values.  Others (3, 5,
-// 6): column-major blocks, lane r holds block row r.
-template <int BS> struct WaveDim {
+// blocks, lane l of a block's G holds pieces q * G + l of V values, those of PR
+// block rows.  Others (3, 5, 6): column-major blocks, lane r holds block row r.
+// A step is bound by what the load / store unit moves: the lanes that hold
+// different rows read the same operands again, so a block is spread over as few
+// lanes as its registers allow.  8 x 8 over 16 lanes, two rows each, two items
+// side by side, against a warp an item and two items in turn: 64^3 application
+// 321 -> 300 us, 160 x 160 (IChol0) 298 -> 267, batched sweeps with 4
+// right-hand sides 258 -> 175 us.  16 x 16 in one warp, four rows a lane in
+// FP64, against two warps: 48^3 363 -> 351 us, 80 x 80 (IChol0) 1159 -> 607.  With
+// several right-hand sides the registers do not suffice for that.
+template <int BS, int R = 1> struct WaveDim {
   static constexpr bool kChunk = (BS & (BS - 1)) == 0;
-  static constexpr int G = BS == 1 ? 1 : BS == 2 ? 2 : BS == 3 ? 4 : BS < 8 ? 8 : 32;  // lanes of a warp per item
-  static constexpr int WPI = BS == 16 ? 2 : 1;                                         // warps per item
+  static constexpr int G = BS == 1 ? 1 : BS == 2 ? 2 : BS == 3 ? 4 : BS < 8 ? 8 : BS == 8 ? 16 : 32;  // lanes of a warp per item
+  static constexpr int WPI = BS == 16 && R > 1 ? 2 : 1;                               // warps per item
   static constexpr int IPW = 32 / G;                                                   // items side by side in a warp
   static constexpr bool kItemMajor = BS >= 4;                                          // order of a step's blocks
-  static constexpr int IPG = BS == 8 ? 2 : 1;                               // items one after another
-  static constexpr int W = kWaveWarps * IPW / WPI * IPG;
+  static constexpr int W = kWaveWarps * IPW / WPI;
   static constexpr int ECAP = W >= 128 ? 64 : W >= 64 ? 32 : W >= 16 ? 16 : 8;
 };
 // External rows of a step with R right-hand sides: with more than one, what the
@@ -74,7 +80,7 @@ template <int BS, int R> constexpr int wave_ecap() { return R == 1 ? WaveDim<BS>
 
 template <int BS, int R> inline WaveShape wave_shape_of() {
   WaveShape s;
-  s.W = WaveDim<BS>::W;
+  s.W = WaveDim<BS, R>::W;
   s.ecap = wave_ecap<BS, R>();
   s.ring = kRing;
   s.slots = kSlots;
@@ -82,8 +88,8 @@ template <int BS, int R> inline WaveShape wave_shape_of() {
   return s;
 }
 
-template <int BS, typename VT> struct WaveMap : WaveDim<BS> {
-  using D = WaveDim<BS>;
+template <int BS, typename VT, int R> struct WaveMap : WaveDim<BS, R> {
+  using D = WaveDim<BS, R>;
   static constexpr int V = !D::kChunk ? BS : BS == 1 ? 1 : BS < 16 ? 2 : sizeof(VT) == 8 ? 2 : 4;
   static constexpr int CPR = D::kChunk ? BS / V : 1;                                  // lanes per block row
   static constexpr int PR = D::kChunk ? BS * BS / V / (D::G * D::WPI) : 1;            // block rows per lane
@@ -96,11 +102,11 @@ template <int BS, typename VT> struct WaveMap : WaveDim<BS> {
 __host__ __device__ constexpr int wave_ld_of(int rw) { return (rw + 1) / 2 * 2; }
 
 template <int BS, typename VT, bool HAS_D, int NE, int R> struct WaveCfg {
-  using M = WaveMap<BS, VT>;
+  using M = WaveMap<BS, VT, R>;
   static constexpr int RW = R * BS;             // values of a vector row
   static constexpr int LD = wave_ld_of(RW);      // its stride in shared memory and in item order
   static constexpr int NB = NE + (HAS_D ? 1 : 0);
-  static constexpr int kRegs = NB * M::NV * M::IPG * (int)sizeof(VT) / 4;  // registers of a step's blocks (at least)
+  static constexpr int kRegs = NB * M::NV * (int)sizeof(VT) / 4;  // registers of a step's blocks (at least)
   static constexpr int DEPTH = kRegs * 2 <= 36 ? 2 : 1;
   static constexpr int LOOK = 2 * DEPTH;  // steps ahead whose headers and records are staged
   static_assert(LOOK + 2 < kSlots, "headers of the steps read ahead are staged");
@@ -110,6 +116,10 @@ template <int BS, typename VT, bool HAS_D, int NE, int R> struct WaveCfg {
   static constexpr int OFF_HDR = OFF_REC + kSlots * M::W * 16;  // {first item, items} of every staged step
   static constexpr int OFF_BAR = OFF_HDR + kSlots * 8;
   static constexpr int kSmem = OFF_BAR + 3 * kSlots * 8;
+  // three turns of polls in flight keep up with the short steps of small blocks
+  // (24 x 20 rows of 2 x 2 blocks 42.7 -> 39.4 us, 40 x 36 x 44 of 4 x 4 133 -> 125);
+  // larger ones need the registers (64^3 of 8 x 8: 321 -> 327 us with three)
+  static constexpr int kFetchWarps = R == 1 && BS <= 4 ? 3 : 2;
   static constexpr int kThreads = (2 * kWaveWarps + 2 + kFetchWarps) * 32;
   static_assert(kSmem <= 226 * 1024, "a CTA's vector rows do not fit shared memory");
 };
@@ -269,9 +279,9 @@ template <int V> __device__ __forceinline__ void wave_vec(const double* p, doubl
 
 template <int BS, typename VT, bool HAS_D, int NE, int R>
 __global__ void __launch_bounds__(WaveCfg<BS, VT, HAS_D, NE, R>::kThreads, 1) k_wave(const WaveP<VT> p) {
-  using M = WaveMap<BS, VT>;
+  using M = WaveMap<BS, VT, R>;
   using C = WaveCfg<BS, VT, HAS_D, NE, R>;
-  constexpr int RW = C::RW, LD = C::LD, W = M::W, DEPTH = C::DEPTH, NB = C::NB, V = M::V, PR = M::PR, NV = M::NV, IPG = M::IPG;
+  constexpr int RW = C::RW, LD = C::LD, W = M::W, DEPTH = C::DEPTH, NB = C::NB, V = M::V, PR = M::PR, NV = M::NV;
   constexpr int B2 = BS * BS, NCW = 2 * kWaveWarps, LOOK = C::LOOK, kBarThreads = (NCW + 1) * 32;
   extern __shared__ __align__(128) unsigned char wv_smem[];
   __shared__ int s_task;
@@ -318,20 +328,26 @@ __global__ void __launch_bounds__(WaveCfg<BS, VT, HAS_D, NE, R>::kThreads, 1) k_
     if (warp < NCW) {
       // ------------------------------------------------------------ compute
       const int set = warp / kWaveWarps, w = warp % kWaveWarps;
-      const int k0 = M::WPI == 2 ? w >> 1 : w * M::IPW + lane / M::G;  // first item; the others W / IPG apart
+      const int k0 = M::WPI == 2 ? w >> 1 : w * M::IPW + lane / M::G;  // the lane's item
       const int gl = lane % M::G;
       const int half = M::WPI == 2 ? w & 1 : 0;
       const int rr = M::kChunk ? half * (BS / 2) + gl / M::CPR : gl;  // first block row of the lane
       const bool has_row = M::kChunk || gl < BS;
       const int r0 = has_row ? rr : BS - 1;
       const int c0 = M::kChunk ? gl % M::CPR * V : 0;
-      // the block row a lane ends up with after the reduction, and whether it
-      // is the lane that writes it
-      const int fr = PR == 2 && (gl & (M::CPR / 2)) ? r0 + M::RPP : r0;
-      const bool owner = has_row && (gl & ((PR == 2 ? M::CPR / 2 : M::CPR) - 1)) == 0;
+      // the block row and the first right-hand side that a lane ends up with
+      // after the reduction, and whether it is the lane that writes them
+      constexpr int REST = M::CPR / PR;                   // lanes that share a row once each has one
+      constexpr bool SPLIT = R > 1 && REST > 1 && BS < 16;  // the last exchange divides the right-hand sides
+      constexpr int RL = SPLIT ? R / 2 : R;
+      int fr = r0;
+      if constexpr (PR == 4) fr += (gl & (M::CPR / 2) ? 2 * M::RPP : 0) + (gl & (M::CPR / 4) ? M::RPP : 0);
+      if constexpr (PR == 2) fr += gl & (M::CPR / 2) ? M::RPP : 0;
+      const int fq = (SPLIT && (gl & 1) ? RL * BS : 0) + fr;
+      const bool owner = has_row && (gl & (REST - 1) & ~(SPLIT ? 1 : 0)) == 0;
       using Piece = WavePiece<VT, M::VP>;
       constexpr int NP = NV / M::VP;
-      Piece blk[DEPTH][IPG][NB][NP];
+      Piece blk[DEPTH][NB][NP];
       int cnt[DEPTH];
       const VT* const lane_vals = p.vals + (int64_t)k0 * (M::kItemMajor ? NB * B2 : B2) +
                                   (M::kChunk ? half * (B2 / 2) + gl * V : r0);
@@ -339,103 +355,102 @@ __global__ void __launch_bounds__(WaveCfg<BS, VT, HAS_D, NE, R>::kThreads, 1) k_
       // step's blocks (W items lie past the last one): a conditional load
       // would be merged with the registers' old contents by a copy that waits
       // for it.  Past the end the last step is read again.
-      auto read_ahead = [&](int t, Piece (&b)[IPG][NB][NP], int& n) {
+      auto read_ahead = [&](int t, Piece (&b)[NB][NP], int& n) {
         const int2 hd = *reinterpret_cast<const int2*>(wv_smem + C::OFF_HDR + min(t, T - 1) % kSlots * 8);
         n = t < T ? hd.y : 0;
         const VT* src = lane_vals;
         if constexpr (M::kItemMajor) src += (int64_t)hd.x * (NB * B2);
         else src += (int64_t)hd.x * NB * B2;
 #pragma unroll
-        for (int j = 0; j < IPG; ++j)
+        for (int e = 0; e < NB; ++e) {
+          const VT* be = src + (M::kItemMajor ? e : e * hd.y) * B2;
 #pragma unroll
-          for (int e = 0; e < NB; ++e) {
-            const VT* be = src;
-            if constexpr (!M::kItemMajor) be += e * hd.y * B2;
-#pragma unroll
-            for (int q = 0; q < NP; ++q)
-              b[j][e][q].load(be + (M::kItemMajor ? (j * (W / IPG) * NB + e) * B2 : j * (W / IPG) * B2) +
-                              q * (M::kChunk ? M::G * V : BS));
-          }
-      };
-      unsigned op[IPG][4];  // byte offsets of the lane's operands in the set's next step
-      int row[IPG];         // the row an item completes, -1: none, -2: no item
-      const unsigned c8 = c0 * 8u;
-      auto decode = [&](int t, int n) {
-#pragma unroll
-        for (int j = 0; j < IPG; ++j) {
-          const int4 rc = reinterpret_cast<const int4*>(wv_smem + C::OFF_REC + k0 * 16)[t % kSlots * W + j * (W / IPG)];
-          op[j][0] = ((unsigned)rc.x & 0xffffu) * (LD * 8u) + c8;
-          op[j][1] = ((unsigned)rc.x >> 16) * (LD * 8u) + c8;
-          op[j][2] = ((unsigned)rc.y & 0xffffu) * (LD * 8u) + c8;
-          op[j][3] = ((unsigned)rc.y >> 16) * (LD * 8u) + c8;
-          row[j] = k0 + j * (W / IPG) < n ? rc.z : -2;
+          for (int q = 0; q < NP; ++q) b[e][q].load(be + q * (M::kChunk ? M::G * V : BS));
         }
       };
-      double* const lane_out = vec + k0 * LD + fr;
+      unsigned op[4];  // byte offsets of the lane's operands in the set's next step
+      int row;         // the row an item completes, -1: none, -2: no item
+      const unsigned c8 = c0 * 8u;
+      auto decode = [&](int t, int n) {
+        const int4 rc = reinterpret_cast<const int4*>(wv_smem + C::OFF_REC + k0 * 16)[t % kSlots * W];
+        op[0] = ((unsigned)rc.x & 0xffffu) * (LD * 8u) + c8;
+        op[1] = ((unsigned)rc.x >> 16) * (LD * 8u) + c8;
+        op[2] = ((unsigned)rc.y & 0xffffu) * (LD * 8u) + c8;
+        op[3] = ((unsigned)rc.y >> 16) * (LD * 8u) + c8;
+        row = k0 < n ? rc.z : -2;
+      };
+      double* const lane_out = vec + k0 * LD + fq;
       named_sync<kBarThreads>(3);  // the first steps' records are there
 #pragma unroll
       for (int d = 0; d < DEPTH; ++d) read_ahead(set + 2 * d, blk[d], cnt[d]);
       if (set < T) decode(set, cnt[0]);
       if (set == 1) named_arrive<kBarThreads>(1);
-      auto one = [&](int t, Piece (&b)[IPG][NB][NP], int& n, const int& n_next) {
+      auto one = [&](int t, Piece (&b)[NB][NP], int& n, const int& n_next) {
         // the earlier steps' rows and this step's staged operands are there
         named_sync<kBarThreads>(1 + set);
-        double out[IPG][R];
+        double out[RL];
+        double sum[R];
 #pragma unroll
-        for (int j = 0; j < IPG; ++j) {
+        for (int q = 0; q < R; ++q) {
+          double acc[NB][PR];
 #pragma unroll
-          for (int q = 0; q < R; ++q) {
-            double acc[NB][PR];
-#pragma unroll
-            for (int e = 0; e < NB; ++e) {
-              double v[V];
-              wave_vec<V>(reinterpret_cast<const double*>(wv_smem + op[j][HAS_D ? e : e + 1]) + q * BS, v);
-#pragma unroll
-              for (int i = 0; i < PR; ++i) {
-                auto val = [&](int c) { return b[j][e][(i * V + c) / M::VP].get((i * V + c) % M::VP); };
-                double s = val(0) * v[0];
-#pragma unroll
-                for (int c = 1; c < V; ++c) s = fma(val(c), v[c], s);
-                acc[e][i] = s;
-              }
-            }
-            double s[PR];
+          for (int e = 0; e < NB; ++e) {
+            double v[V];
+            wave_vec<V>(reinterpret_cast<const double*>(wv_smem + op[HAS_D ? e : e + 1]) + q * BS, v);
 #pragma unroll
             for (int i = 0; i < PR; ++i) {
-              s[i] = acc[0][i] + acc[1][i];
-              if constexpr (NB == 3) s[i] += acc[2][i];
-              if constexpr (NB == 4) s[i] += acc[2][i] + acc[3][i];
-            }
-            // sum over the CPR lanes of a block row; a lane with two rows
-            // hands one of them over in the first exchange
-            int o = M::CPR / 2;
-            if constexpr (PR == 2) {
-              const bool hi = (gl & o) != 0;
-              const double give = hi ? s[0] : s[1];
-              s[0] = (hi ? s[1] : s[0]) + __shfl_xor_sync(0xffffffffu, give, o);
-              o >>= 1;
-            }
+              auto val = [&](int c) { return b[e][(i * V + c) / M::VP].get((i * V + c) % M::VP); };
+              double s = val(0) * v[0];
 #pragma unroll
-            for (; o >= 1; o >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
-            out[j][q] = s[0];
-            if constexpr (!HAS_D) out[j][q] += reinterpret_cast<const double*>(wv_smem + op[j][0])[q * BS + fr - c0];
+              for (int c = 1; c < V; ++c) s = fma(val(c), v[c], s);
+              acc[e][i] = s;
+            }
           }
+          double s[PR];
+#pragma unroll
+          for (int i = 0; i < PR; ++i) {
+            s[i] = acc[0][i] + acc[1][i];
+            if constexpr (NB == 3) s[i] += acc[2][i];
+            if constexpr (NB == 4) s[i] += acc[2][i] + acc[3][i];
+          }
+          // sum over the CPR lanes of a block row; a lane with several rows
+          // hands half of them over in an exchange until one is left
+          int o = M::CPR / 2;
+#pragma unroll
+          for (int n = PR / 2; n >= 1; n >>= 1, o >>= 1) {
+            const bool hi = (gl & o) != 0;
+#pragma unroll
+            for (int i = 0; i < n; ++i) {
+              const double give = hi ? s[i] : s[i + n];
+              s[i] = (hi ? s[i + n] : s[i]) + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+          }
+#pragma unroll
+          for (; o >= (SPLIT ? 2 : 1); o >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
+          sum[q] = s[0];
         }
 #pragma unroll
-        for (int j = 0; j < IPG; ++j)
-          if (owner && row[j] >= -1) {
-            double* xo = lane_out + (t % kRing * W + j * (W / IPG)) * LD;
-#pragma unroll
-            for (int q = 0; q < R; ++q) xo[q * BS] = out[j][q];
+        for (int q = 0; q < RL; ++q) {
+          if constexpr (SPLIT) {
+            const bool hi = (gl & 1) != 0;
+            const double give = hi ? sum[q] : sum[q + RL];
+            out[q] = (hi ? sum[q + RL] : sum[q]) + __shfl_xor_sync(0xffffffffu, give, 1);
+          } else {
+            out[q] = sum[q];
           }
+          if constexpr (!HAS_D) out[q] += reinterpret_cast<const double*>(wv_smem + op[0])[q * BS + fq - c0];
+        }
+        if (owner && row >= -1) {
+          double* xo = lane_out + t % kRing * W * LD;
+#pragma unroll
+          for (int q = 0; q < RL; ++q) xo[q * BS] = out[q];
+        }
         if (t + 1 < T) named_arrive<kBarThreads>(1 + (set ^ 1));
+        if (owner && row >= 0) {
+          double* xg = p.x + (int64_t)row * p.xs + fq;
 #pragma unroll
-        for (int j = 0; j < IPG; ++j)
-          if (owner && row[j] >= 0) {
-            double* xg = p.x + (int64_t)row[j] * p.xs + fr;
-#pragma unroll
-            for (int q = 0; q < R; ++q) st_publish(xg + q * BS, out[j][q]);
-          }
+          for (int q = 0; q < RL; ++q) st_publish(xg + q * BS, out[q]);
+        }
         read_ahead(t + 2 * DEPTH, b, n);
         if (t + 2 < T) decode(t + 2, n_next);
       };
@@ -489,7 +504,7 @@ __global__ void __launch_bounds__(WaveCfg<BS, VT, HAS_D, NE, R>::kThreads, 1) k_
       // -------------------------------------------------------------- fetch
       // the rows of a step are named three turns of this warp ahead
       constexpr int NX = (C::ECAP * RW + 31) / 32;
-      constexpr int F = kFetchWarps;
+      constexpr int F = C::kFetchWarps;
       const int* hp = reinterpret_cast<const int*>(p.step + t0) + 1;
       struct Turn {
         int er[NX];    // the rows of its values
