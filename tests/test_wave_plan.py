@@ -126,6 +126,18 @@ def test_steps_follow_the_wavefront(lib):
     assert rc == 0 and stats[0] == 1 and stats[1] == 127
 
 
+@pytest.mark.parametrize("dims,supers", [((80, 80), 10), ((20, 40), 5), ((6, 90), 1), ((9, 8), 1)])
+def test_super_tasks_of_a_2d_grid(lib, dims, supers):
+    """W = 8: long lines 8 to a super-task, a line's step after the one before;
+    short lines as many as reach 1024 rows."""
+    n, deps = grid(dims)
+    rc, x, ref, stats = run(lib, n, deps, 16, True, True, SHAPES[16])
+    assert rc == 0 and np.abs(x - ref).max() <= 1e-13 * np.abs(ref).max()
+    assert stats[0] == supers
+    if supers > 1:
+        assert stats[1] == supers * (dims[0] + 7)
+
+
 def test_not_triangular_is_refused(lib):
     ptr, col = np.array([0, 1, 1], np.int32), np.array([1], np.int32)
     one = np.zeros(16)
