@@ -25,13 +25,14 @@
 //     the barrier and take no issue slots from the warps that poll (a failed
 //     mbarrier test returns at once, so 16 polling warps would).
 //
-// What bounds it: on small and thin systems the number of dependency levels
-// times the time of a step (about 0.3 us: barrier, shared-memory operands,
-// multiply-adds and lane reduction, and the load / store unit, which moves
-// every block and operand); on large ones that and HBM, every block being read
-// once.  One application (two sweeps and the preparation), measured against
-// the kernels this replaced (level-ordered polling rows; for 8 x 8 and 16 x 16
-// blocks chains that polled shared memory):
+// What bounds it: the number of dependency levels times the time of a step
+// (about 0.3 us: barrier, shared-memory operands, multiply-adds and lane
+// reduction, one after another), on large systems too: at 64^3 with 8 x 8 blocks
+// DRAM is 37 to 44 % busy and the issue slots 20 %, and two stalls of three are
+// at the step barrier.  Every block is read once.  One application (two sweeps
+// and the preparation), measured against the kernels this replaced
+// (level-ordered polling rows; for 8 x 8 and 16 x 16 blocks chains that polled
+// shared memory):
 //   ILU0   64^3, 8 x 8           377 -> 300 us (3.2 TB/s)
 //   ILU0   48^3, 16 x 16         720 -> 351 us
 //   IChol0 300 x 257, 4 x 4     4825 -> 360 us (556 levels, twice)
@@ -57,9 +58,9 @@ constexpr int kRing = 8;        // steps whose results stay in shared memory
 // Lanes and CTA shape of a block size.  Sizes 1, 2, 4, 8, 16: row-major
 // blocks, lane l of a block's G holds pieces q * G + l of V values, those of PR
 // block rows.  Others (3, 5, 6): column-major blocks, lane r holds block row r.
-// A step is bound by what the load / store unit moves: the lanes that hold
-// different rows read the same operands again, so a block is spread over as few
-// lanes as its registers allow.  8 x 8 over 16 lanes, two rows each, two items
+// A step begins with the operand reads of its 8 warps all at once, and the
+// lanes that hold different rows of a block read the same operands again, so a
+// block is spread over as few lanes as its registers allow.  8 x 8 over 16 lanes, two rows each, two items
 // side by side, against a warp an item and two items in turn: 64^3 application
 // 321 -> 300 us, 160 x 160 (IChol0) 298 -> 267, batched sweeps with 4
 // right-hand sides 258 -> 175 us.  16 x 16 in one warp, four rows a lane in

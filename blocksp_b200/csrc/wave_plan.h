@@ -266,8 +266,7 @@ inline bool wave_plan(int n, bool ascending, const WaveShape& S, bool has_d, con
   for (int sid : order) {
     const Sup& sp = sups[sid];
     P.n_levels = std::max(P.n_levels, sp.level + 1);
-    st.clear();
-    ext.clear();
+    size_t used = 0;  // steps of this super-task: their lists keep what they held room for
     size_t hint = 0;  // steps before it are full
     for (int r : sp.rows) {
       ord.clear();
@@ -278,14 +277,16 @@ inline bool wave_plan(int n, bool ascending, const WaveShape& S, bool has_d, con
         ord.emplace_back(s, t);
         lo = std::max(lo, s + 1);
       }
-      std::stable_sort(ord.begin(), ord.end(), [](auto& a, auto& b) { return a.first < b.first; });
+      // few entries: by insertion (a stable sort would allocate for every row)
+      for (size_t a = 1; a < ord.size(); ++a)
+        for (size_t b = a; b > 0 && ord[b].first < ord[b - 1].first; --b) std::swap(ord[b], ord[b - 1]);
       const int ne = (int)ord.size();
       seg.clear();
       for (int f = 0; f == 0 || f < ne; f += NE) seg.emplace_back(f, std::min(ne - f, NE));
       const int ns = (int)seg.size();
       // whether the external rows of a segment at step s fit
       auto ext_fit = [&](int s, const std::pair<int, int>& sg) {
-        const int have = s < (int)ext.size() ? (int)ext[s].size() : 0;
+        const int have = s < (int)used ? (int)ext[s].size() : 0;
         int need = 0;
         for (int u = 0; u < sg.second; ++u) {
           const auto& o = ord[sg.first + u];
@@ -293,22 +294,26 @@ inline bool wave_plan(int n, bool ascending, const WaveShape& S, bool has_d, con
         }
         return need == 0 || have + need <= S.ecap;
       };
-      while (hint < st.size() && (int)st[hint].size() >= S.W) ++hint;
+      while (hint < used && (int)st[hint].size() >= S.W) ++hint;
       at.assign(ns, 0);
       for (int base = std::max({lo - ns + 1, 0, (int)hint});; ++base) {
         bool good = true;
         int s = base;
         for (int k = 0; k < ns && good; ++k) {
           for (int u = 0; u < seg[k].second; ++u) s = std::max(s, ord[seg[k].first + u].first + 1);
-          while ((s < (int)st.size() && (int)st[s].size() >= S.W) || !ext_fit(s, seg[k])) ++s;
+          while ((s < (int)used && (int)st[s].size() >= S.W) || !ext_fit(s, seg[k])) ++s;
           if (k > 0 && s - at[k - 1] > lag) good = false;
           at[k] = s++;
         }
         if (good) break;
       }
-      if (at[ns - 1] >= (int)st.size()) {
-        st.resize(at[ns - 1] + 1);
-        ext.resize(at[ns - 1] + 1);
+      for (; (int)used <= at[ns - 1]; ++used) {
+        if (used == st.size()) {
+          st.emplace_back();
+          ext.emplace_back();
+        }
+        st[used].clear();
+        ext[used].clear();
       }
       int prev_item = 0;
       for (int k = 0; k < ns; ++k) {
@@ -342,7 +347,7 @@ inline bool wave_plan(int n, bool ascending, const WaveShape& S, bool has_d, con
       r_item[r] = prev_item;
     }
     // flatten
-    for (size_t s = 0; s < st.size(); ++s) {
+    for (size_t s = 0; s < used; ++s) {
       P.step.push_back({(int32_t)P.rec.size(), (int32_t)P.ext_row.size()});
       for (const Item& it : st[s]) {
         P.rec.push_back({(uint32_t)it.base | (uint32_t)it.c[0] << 16, (uint32_t)it.c[1] | (uint32_t)it.c[2] << 16,
