@@ -327,6 +327,7 @@ __global__ void __launch_bounds__(32) k_gm_ls(GPtrs g, int max_iters) {
   double res = 0.0;
   if (j + 2 <= kLsRows) {
     for (int i = lane; i <= j + 1; i += 32) col[i] = g.H[i * g.m + j];
+    __syncwarp();  // lane 0 reads the column next; the first one has no rotations to wait for
     for (int t0 = 0; t0 < nrot; t0 += kLsRots) {
       const int n = min(kLsRots, nrot - t0);
       __syncwarp();
