@@ -427,7 +427,7 @@ struct BContP {
   int n_groups;
   int* counter;   // iterations executed
   int* running;   // 1 while any pair runs (read by the host-driven mode)
-  int cap;        // hard bound on iterations
+  const BOpts* opts;        // this call's limits: the graph is kept from one call to the next
   const DevStatus* dev_st;  // device error word: a failed sweep ends the loop
 };
 
@@ -444,7 +444,8 @@ __global__ void k_bt_continue(BContP c, cudaGraphConditionalHandle hnd, int use_
     *c.counter = it;
     // a sweep that timed out (or any other device failure) ends the loop at
     // once: the host reads the status after the launch
-    const int run = any && it < c.cap && *reinterpret_cast<const volatile int*>(&c.dev_st->code) == 0;
+    const int run = any && (int64_t)it < (int64_t)c.opts->max_iters + 2 &&
+                    *reinterpret_cast<const volatile int*>(&c.dev_st->code) == 0;
     *c.running = run;
     if (use_cond) cudaGraphSetConditional(hnd, run ? 1u : 0u);
   }
@@ -639,7 +640,7 @@ int enqueue_group(bsp_batch_s* B, BatchGroup& g, const Kernels& k, cudaStream_t 
   return BSP_OK;
 }
 
-BContP cont_params(bsp_batch_s* B, int max_iters) {
+BContP cont_params(bsp_batch_s* B) {
   BContP c{};
   c.n_groups = (int)B->groups.size();
   for (int i = 0; i < c.n_groups; ++i) {
@@ -648,14 +649,14 @@ BContP cont_params(bsp_batch_s* B, int max_iters) {
   }
   c.counter = B->counter.get();
   c.running = B->counter.get() + 1;
-  c.cap = max_iters + 2;
+  c.opts = B->opts.get();
   c.dev_st = B->h->ws.status.get();
   return c;
 }
 
 // Fork the phase over the group streams and join back into `s`; count: kernels.
 int enqueue_phase(bsp_batch_s* B, const std::vector<Kernels>& ks, cudaStream_t s, bool init,
-                  cudaGraphConditionalHandle hnd, int use_cond, int max_iters, int64_t& count) {
+                  cudaGraphConditionalHandle hnd, int use_cond, int64_t& count) {
   int n = 0;
   BSP_CUDA_TRY(cudaEventRecord(B->fork, s));
   for (size_t gi = 0; gi < B->groups.size(); ++gi) {
@@ -664,7 +665,7 @@ int enqueue_phase(bsp_batch_s* B, const std::vector<Kernels>& ks, cudaStream_t s
     BSP_CUDA_TRY(cudaEventRecord(B->join[gi], B->gs[gi]));
     BSP_CUDA_TRY(cudaStreamWaitEvent(s, B->join[gi], 0));
   }
-  k_bt_continue<<<1, 256, 0, s>>>(cont_params(B, max_iters), hnd, use_cond, init ? 0 : 1);
+  k_bt_continue<<<1, 256, 0, s>>>(cont_params(B), hnd, use_cond, init ? 0 : 1);
   BSP_CUDA_TRY(cudaPeekAtLastError());
   count = n + 1;
   return BSP_OK;
@@ -808,7 +809,7 @@ void destroy_graphs(bsp_batch_s* B) {
 
 // Captures the solve.  mode 0: init + while(body) in one graph; mode 1: init
 // and body as two graphs, the body replayed by the host.
-int build_graphs(bsp_batch_s* B, const std::vector<Kernels>& ks, int mode, int max_iters) {
+int build_graphs(bsp_batch_s* B, const std::vector<Kernels>& ks, int mode) {
   destroy_graphs(B);
   cudaStream_t s = B->cap;
   if (mode == 0) {
@@ -818,7 +819,7 @@ int build_graphs(bsp_batch_s* B, const std::vector<Kernels>& ks, int mode, int m
     // the loop body runs at least once; from then on its last kernel decides
     BSP_CUDA_TRY(cudaGraphConditionalHandleCreate(&hnd, graph, 1, cudaGraphCondAssignDefault));
     BSP_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
-    BSP_TRY(enqueue_phase(B, ks, s, true, hnd, 0, max_iters, B->init_kernels));
+    BSP_TRY(enqueue_phase(B, ks, s, true, hnd, 0, B->init_kernels));
     BSP_CUDA_TRY(cudaStreamEndCapture(s, &init));
     cudaGraphNode_t init_node, cond_node;
     BSP_CUDA_TRY(cudaGraphAddChildGraphNode(&init_node, graph, nullptr, 0, init));
@@ -831,7 +832,7 @@ int build_graphs(bsp_batch_s* B, const std::vector<Kernels>& ks, int mode, int m
     BSP_CUDA_TRY(cudaGraphAddNode(&cond_node, graph, &init_node, 1, &cp));
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     BSP_CUDA_TRY(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-    BSP_TRY(enqueue_phase(B, ks, s, false, hnd, 1, max_iters, B->body_kernels));
+    BSP_TRY(enqueue_phase(B, ks, s, false, hnd, 1, B->body_kernels));
     BSP_CUDA_TRY(cudaStreamEndCapture(s, &body));
     const cudaError_t e = cudaGraphInstantiate(&B->exec, graph, 0);
     cudaGraphDestroy(graph);
@@ -839,10 +840,10 @@ int build_graphs(bsp_batch_s* B, const std::vector<Kernels>& ks, int mode, int m
   } else {
     cudaGraph_t init = nullptr, body = nullptr;
     BSP_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
-    BSP_TRY(enqueue_phase(B, ks, s, true, 0, 0, max_iters, B->init_kernels));
+    BSP_TRY(enqueue_phase(B, ks, s, true, 0, 0, B->init_kernels));
     BSP_CUDA_TRY(cudaStreamEndCapture(s, &init));
     BSP_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
-    BSP_TRY(enqueue_phase(B, ks, s, false, 0, 0, max_iters, B->body_kernels));
+    BSP_TRY(enqueue_phase(B, ks, s, false, 0, 0, B->body_kernels));
     BSP_CUDA_TRY(cudaStreamEndCapture(s, &body));
     cudaError_t e = cudaGraphInstantiate(&B->exec, init, 0);
     if (e == cudaSuccess) e = cudaGraphInstantiate(&B->exec_body, body, 0);
@@ -1027,7 +1028,7 @@ int bsp_batch_pcg_dev(bsp_handle_t h, bsp_batch_t B, int nrhs, const double* b, 
   if (rebuild) {
     for (size_t gi = 0; gi < B->groups.size(); ++gi)
       if (!B->groups[gi].tuned || o->retune) BSP_TRY(autotune(B, B->groups[gi], ks[gi]));
-    BSP_TRY(build_graphs(B, ks, o->mode, o->max_iters));
+    BSP_TRY(build_graphs(B, ks, o->mode));
     B->graph_R = nrhs;
     B->graph_hist = hist_cap;
     B->graph_mode = o->mode;
