@@ -21,6 +21,7 @@
 // slice, at most 7 (5 complex ones): the sums of a step then fit one value per
 // lane.
 #pragma once
+#include "per_device.h"
 #include "reduce.cuh"
 #include "sentinel.cuh"
 #include "stage.cuh"
@@ -276,14 +277,14 @@ __global__ void __launch_bounds__(TH, 1) k_mgs(const MgsP p) {
 template <int TH, int NPT, int B, int U, bool CX> int launch_mgs_t(bsp_handle_s* h, MgsP& p) {
   constexpr size_t smem = (size_t)B * TH * NPT * sizeof(double);
   static_assert(smem <= kMgsSmem, "the slices of a block of vectors do not fit shared memory");
-  static bool ok = false;
+  static PerDevice ready;
   auto kern = k_mgs<TH, NPT, B, U, CX>;
-  if (!ok) {
+  if (!ready.has(h->device)) {
     BSP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     BSP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TH, smem));
     if (per_sm < 1) return 1;
-    ok = true;
+    ready.set(h->device);
   }
   p.slice = (int64_t)TH * NPT;
   void* args[] = {&p};

@@ -39,8 +39,10 @@
 // rows i < k in increasing i, exactly the sequence of updates the reference's
 // right-looking loop applies to each block (k, j), so the factors are the same.
 #include <algorithm>
+#include <atomic>
 #include <numeric>
 #include "blockops.cuh"
+#include "per_device.h"
 #include "precond.hpp"
 #include "reduce.cuh"
 #include "sentinel.cuh"
@@ -1161,11 +1163,13 @@ static int run_factor(bsp_precond_s* pc, int mode, const int* order, const int* 
 template <int BS, typename VT, typename AT, bool TRANS, int POST>
 static int launch_sweep_t(bsp_handle_s* h, const SweepP<VT, AT>& p) {
   constexpr size_t smem = SweepCfg<BS, VT, AT, TRANS, POST>::kSmem;
-  static int per_sm = 0;
-  if (!per_sm) {
+  static PerDevice ready;
+  static std::atomic<int> per_sm{1};  // resident CTAs an SM (every device is the same part)
+  if (!ready.has(h->device)) {
     BSP_CUDA_TRY(cudaFuncSetAttribute(k_sweep<BS, VT, AT, TRANS, POST>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     per_sm = persistent_grid(h, k_sweep<BS, VT, AT, TRANS, POST>, kSweepThreads, smem) / h->num_sms;
+    ready.set(h->device);
   }
   bsp::count_launch(),
       k_sweep<BS, VT, AT, TRANS, POST><<<h->num_sms * per_sm, kSweepThreads, smem, h->stream>>>(p);
@@ -1203,8 +1207,9 @@ static int launch_sweep(bsp_handle_s* h, int bs, SweepP<VT, AT> p, unsigned* tic
   }
 #undef BSP_SWEEP_CASE
   if (!done) {
-    static int grid = 0;
-    if (!grid) grid = persistent_grid(h, k_sweep_generic<VT, AT, TRANS, POST>, kSweepThreads, 0);
+    static std::atomic<int> per_sm{0};
+    if (!per_sm) per_sm = persistent_grid(h, k_sweep_generic<VT, AT, TRANS, POST>, kSweepThreads, 0) / h->num_sms;
+    const int grid = h->num_sms * per_sm;
     p.task_row = nullptr;  // the generic kernel takes one row per ticket
     bsp::count_launch(), k_sweep_generic<VT, AT, TRANS, POST><<<grid, kSweepThreads, 0, h->stream>>>(p, bs);
   }

@@ -45,6 +45,7 @@
 // step), one set of compute warps (0.42 us a step on 2D grids instead of 0.3),
 // prefetching the blocks into L2 further ahead (no gain).
 #pragma once
+#include "per_device.h"
 #include "sentinel.cuh"
 #include "stage.cuh"
 #include "sweep_wave.hpp"
@@ -608,11 +609,11 @@ template <typename VT> WaveP<VT> wave_params(bsp_handle_s* h, const WaveSym& S, 
 template <int BS, typename VT, bool HAS_D, int NE, int R>
 int wave_launch(bsp_handle_s* h, const WaveP<VT>& p, cudaStream_t stream) {
   using C = WaveCfg<BS, VT, HAS_D, NE, R>;
-  static bool ready = false;
+  static PerDevice ready;
   auto kern = k_wave<BS, VT, HAS_D, NE, R>;
-  if (!ready) {
+  if (!ready.has(h->device)) {
     BSP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem));
-    ready = true;
+    ready.set(h->device);
   }
   const int grid = p.n_super < h->num_sms ? (p.n_super < 1 ? 1 : p.n_super) : h->num_sms;
   kern<<<grid, C::kThreads, C::kSmem, stream>>>(p);
