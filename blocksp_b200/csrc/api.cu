@@ -64,6 +64,9 @@ cudaError_t pool_alloc(void** p, size_t bytes, size_t* cap, int* device) {
       pool_trim_locked(P, dev);
     }
     e = cudaMalloc(p, bytes);
+    // the caller gets the error as a value: left pending, the next launch check
+    // would report it as its own
+    if (e != cudaSuccess) cudaGetLastError();
   }
   *cap = bytes;
   return e;

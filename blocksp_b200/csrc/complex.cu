@@ -217,9 +217,14 @@ int pgmres_complex_solve(bsp_handle_s* h, bsp_matrix_s* A, bsp_precond_s* pc, co
     BSP_TRY(bsmv_launch(A, 1, 0, BSP_F64, 1.0, Q[iter], 0.0, nullptr, w, st));
     if (pc) BSP_TRY(precond_apply(pc, BSP_PREC_F64, w, w));
     // the basis grows by a few vectors at a time where memory allows
-    if ((int)Q.size() < iter + 2)
-      for (int i = (int)Q.size(); i < std::min(iter + 8, cols) && basis(i); ++i) {}
-    if (!basis(iter + 1)) return BSP_OUT_OF_MEMORY;
+    if ((int)Q.size() < iter + 2) {
+      if (!basis(iter + 1)) return BSP_OUT_OF_MEMORY;
+      for (int i = iter + 2; i < std::min(iter + 8, cols); ++i)
+        if (!basis(i)) {
+          record_error("");  // not this solve's: it goes on without looking ahead
+          break;
+        }
+    }
     if ((int)Q.size() > n_tab) {  // its table on the device
       n_tab = (int)Q.size();
       BSP_CUDA_TRY(cudaMemcpyAsync(qtab, Q.data(), n_tab * sizeof(double*), cudaMemcpyHostToDevice, st));

@@ -962,7 +962,7 @@ int pgmres_solve(bsp_handle_s* h, bsp_matrix_s* A, bsp_precond_s* pc, const doub
     // (a column past the end of the solve is not used)
     queued = j + 1 < m && st.tot < o->max_iters && heads.ahead(st);
     if (queued && ensure_basis(j + 3) != BSP_OK) {
-      cudaGetLastError();
+      record_error("");  // not this solve's: it goes on without looking ahead
       queued = false;
     }
     if (queued) BSP_TRY(column(j + 1));
