@@ -711,8 +711,14 @@ int build_sweeps(bsp_batch_s* B, BatchGroup& g, int R) {
   std::vector<int> beg(g.row_off.begin(), g.row_off.end()), iu;
   g.lo = WaveSym{};
   g.up = WaveSym{};
-  BSP_TRY(wave_build(n, g.bs, false, up, true, true, true, beg, R, nullptr, &iu, g.up));
-  BSP_TRY(wave_build(n, g.bs, true, lo, false, true, false, beg, R, &iu, nullptr, g.lo));
+  const WaveShape S = wave_shape(g.bs, R);
+  WavePlan p_lo, p_up;
+  if (!wave_plan(n, false, S, true, up, beg, p_up) || !wave_plan(n, true, S, true, lo, beg, p_lo)) {
+    record_error("batched sweeps: the layout is too long");
+    return BSP_INVALID;
+  }
+  BSP_TRY(wave_upload(std::move(p_up), g.bs, true, true, true, nullptr, &iu, g.up));
+  BSP_TRY(wave_upload(std::move(p_lo), g.bs, false, true, false, &iu, nullptr, g.lo));
   BSP_TRY(wave_gather(B->h, g.lo, BSP_PREC_F64, g.pc->f_vals.get(), g.pc->dinv.get(), g.v_lo));
   BSP_TRY(wave_gather(B->h, g.up, BSP_PREC_F64, g.pc->f_vals.get(), g.pc->dinv.get(), g.v_up));
   return BSP_OK;

@@ -78,6 +78,7 @@ struct Workspace {
 };
 
 struct WaveSym;
+struct StreamSym;
 struct FactorPlan;
 
 // Structure-only analysis behind a preconditioner (sorted factor pattern,
@@ -92,8 +93,9 @@ struct SymbolicCache {
   DevBuf<int> f_ptr, f_col, f_diag, order_lo, order_up, task_lo_row, task_lo_len, task_up_row,
       task_up_len, t_ptr, t_row, a_diag;
   DevBuf<int64_t> d_perm, t_blk;
-  // lock-step layouts of the two sweeps (block sizes their kernel takes)
+  // lock-step or streamed layouts of the two sweeps (sweep_plan.hpp), or none
   std::shared_ptr<WaveSym> wv_lo, wv_up;
+  std::shared_ptr<StreamSym> ss_lo, ss_up;
   // elimination plan of the row-resident factorisation kernel
   std::shared_ptr<FactorPlan> plan;
 };

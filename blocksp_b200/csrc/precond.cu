@@ -47,7 +47,7 @@
 #include "reduce.cuh"
 #include "sentinel.cuh"
 #include "stage.cuh"
-#include "sweep_wave.hpp"
+#include "sweep_plan.hpp"
 
 namespace bsp {
 
@@ -1026,6 +1026,8 @@ static int sym_transfer(bsp_precond_s* pc, SymbolicCache& C, bool save) {
   if (save) {
     C.wv_lo = pc->wv_lo;
     C.wv_up = pc->wv_up;
+    C.ss_lo = pc->ss_lo;
+    C.ss_up = pc->ss_up;
     C.plan = pc->plan;
     C.h_perm = pc->h_perm;
     C.f_nnzb = pc->f_nnzb;
@@ -1037,6 +1039,8 @@ static int sym_transfer(bsp_precond_s* pc, SymbolicCache& C, bool save) {
   } else {
     pc->wv_lo = C.wv_lo;
     pc->wv_up = C.wv_up;
+    pc->ss_lo = C.ss_lo;
+    pc->ss_up = C.ss_up;
     pc->plan = C.plan;
     pc->h_perm = C.h_perm;
     pc->f_nnzb = C.f_nnzb;
@@ -1307,84 +1311,65 @@ static int analyse_factor_structure(bsp_precond_s* pc, bool lower_only) {
   BSP_TRY(upload(pc->f_col, col));
   BSP_TRY(upload(pc->f_diag, diag));
   BSP_TRY(upload(pc->d_perm, perm));
-  // level orders and chain tasks on the sorted structure
-  std::vector<int> order;
-  auto lower_deps = [&](int i, auto&& f) {
-    for (int e = ptr[i]; e < diag[i]; ++e) f(col[e]);
-  };
-  pc->n_lev_lo = level_order(n, true, lower_deps, order);
-  BSP_TRY(upload(pc->order_lo, order));
-  BSP_TRY(make_tasks(pc, true, n, lower_deps));
-  // lock-step layouts of both sweeps (ILU0: unit L, then U with U_ii^-1;
+  // the sweeps are laid out beside the rest (ILU0: unit L, then U with U_ii^-1;
   // IChol0: L with L_ii^-1, then L^T with L_ii^-T)
-  const bool wave = wave_supported(pc->bs);
-  SweepEntries ent;
-  // strictly-lower (lower = true) or strictly-upper entries of the factor
-  auto tri_entries = [&](bool lower) {
-    ent.ptr.assign(n + 1, 0);
-    ent.col.clear();
-    ent.blk.clear();
-    for (int i = 0; i < n; ++i) {
-      const int a = lower ? ptr[i] : diag[i] + 1, b = lower ? diag[i] : ptr[i + 1];
-      for (int e = a; e < b; ++e) {
-        ent.col.push_back(col[e]);
-        ent.blk.push_back(e);
-      }
-      ent.ptr[i + 1] = (int)ent.col.size();
+  SweepPlanner sweeps;
+  SweepEntries &lo = sweeps.lo, &up = sweeps.up;
+  lo.ptr.assign(n + 1, 0);
+  up.ptr.assign(n + 1, 0);
+  lo.col.reserve(col.size());
+  lo.blk.reserve(col.size());
+  for (int i = 0; i < n; ++i) {
+    for (int e = ptr[i]; e < diag[i]; ++e) {
+      lo.col.push_back(col[e]);
+      lo.blk.push_back(e);
+      if (lower_only) up.ptr[col[e] + 1]++;
     }
-  };
-  std::vector<int> up_item;  // per row: the item of the backward sweep that reads it
-  if (!lower_only) {
-    auto upper_deps = [&](int i, auto&& f) {
-      for (int e = diag[i] + 1; e < ptr[i + 1]; ++e) f(col[e]);
-    };
-    pc->n_lev_up = level_order(n, false, upper_deps, order);
-    BSP_TRY(upload(pc->order_up, order));
-    BSP_TRY(make_tasks(pc, false, n, upper_deps));
-    if (wave) {
-      tri_entries(false);
-      pc->wv_up = std::make_shared<WaveSym>();
-      BSP_TRY(wave_build(n, pc->bs, false, ent, false, true, false, {}, 1, nullptr, &up_item, *pc->wv_up));
+    lo.ptr[i + 1] = (int)lo.col.size();
+    if (lower_only) continue;
+    for (int e = diag[i] + 1; e < ptr[i + 1]; ++e) {
+      up.col.push_back(col[e]);
+      up.blk.push_back(e);
     }
-  } else {
+    up.ptr[i + 1] = (int)up.col.size();
+  }
+  if (lower_only) {
     // L^T backward: row i depends on rows j > i with L_ji present
-    std::vector<int> tp(n + 1, 0);
-    for (int j = 0; j < n; ++j)
-      for (int e = ptr[j]; e < diag[j]; ++e) tp[col[e] + 1]++;
-    for (int i = 0; i < n; ++i) tp[i + 1] += tp[i];
-    std::vector<int> trow(tp[n]);
-    std::vector<int64_t> tblk(tp[n]);
-    std::vector<int> fill(tp.begin(), tp.end() - 1);
+    for (int i = 0; i < n; ++i) up.ptr[i + 1] += up.ptr[i];
+    up.col.resize(up.ptr[n]);
+    up.blk.resize(up.ptr[n]);
+    std::vector<int> fill(up.ptr.begin(), up.ptr.end() - 1);
     for (int j = 0; j < n; ++j)
       for (int e = ptr[j]; e < diag[j]; ++e) {
-        const int i = col[e];
-        trow[fill[i]] = j;
-        tblk[fill[i]] = e;
-        fill[i]++;
+        const int p = fill[col[e]]++;
+        up.col[p] = j;
+        up.blk[p] = e;
       }
-    auto trans_deps = [&](int i, auto&& f) {
-      for (int t = tp[i]; t < tp[i + 1]; ++t) f(trow[t]);
+  }
+  sweeps.lo_d = lower_only;
+  sweeps.up_d = true;
+  sweeps.up_trans = sweeps.up_trans_d = lower_only;
+  sweeps.start(n, pc->bs);
+  // level orders and chain tasks on the sorted structure
+  std::vector<int> order;
+  auto deps_of = [](const SweepEntries& E) {
+    return [&E](int i, auto&& f) {
+      for (int t = E.ptr[i]; t < E.ptr[i + 1]; ++t) f(E.col[t]);
     };
-    pc->n_lev_up = level_order(n, false, trans_deps, order);
-    BSP_TRY(upload(pc->order_up, order));
-    BSP_TRY(make_tasks(pc, false, n, trans_deps));
-    if (wave) {
-      ent.ptr = tp;
-      ent.col = trow;
-      ent.blk = tblk;
-      pc->wv_up = std::make_shared<WaveSym>();
-      BSP_TRY(wave_build(n, pc->bs, false, ent, true, true, true, {}, 1, nullptr, &up_item, *pc->wv_up));
-    }
-    BSP_TRY(upload(pc->t_ptr, tp));
-    BSP_TRY(upload(pc->t_row, trow));
-    BSP_TRY(upload(pc->t_blk, tblk));
+  };
+  pc->n_lev_lo = level_order(n, true, deps_of(lo), order);
+  BSP_TRY(upload(pc->order_lo, order));
+  BSP_TRY(make_tasks(pc, true, n, deps_of(lo)));
+  pc->n_lev_up = level_order(n, false, deps_of(up), order);
+  BSP_TRY(upload(pc->order_up, order));
+  BSP_TRY(make_tasks(pc, false, n, deps_of(up)));
+  if (lower_only) {
+    BSP_TRY(upload(pc->t_ptr, up.ptr));
+    BSP_TRY(upload(pc->t_row, up.col));
+    BSP_TRY(upload(pc->t_blk, up.blk));
   }
-  if (wave) {
-    tri_entries(true);
-    pc->wv_lo = std::make_shared<WaveSym>();
-    BSP_TRY(wave_build(n, pc->bs, true, ent, false, lower_only, false, {}, 1, &up_item, nullptr, *pc->wv_lo));
-  }
-  return build_factor_plan(pc, n, ptr, col, diag, lower_only);
+  BSP_TRY(build_factor_plan(pc, n, ptr, col, diag, lower_only));
+  return sweeps.finish(pc->wv_lo, pc->wv_up, pc->ss_lo, pc->ss_up);
 }
 
 // Factor storage for ILU0 / IChol0: the symbolic part from the matrix's cache
@@ -1422,38 +1407,35 @@ static int analyse_diag_structure(bsp_precond_s* pc) {
     std::vector<int> order;
     const auto& rp = A->h_row_ptr;
     const auto& ci = A->h_col_idx;
-    auto lower_deps = [&](int i, auto&& f) {
-      for (int t = rp[i]; t < rp[i + 1]; ++t)
-        if (ci[t] < i) f(ci[t]);
-    };
-    auto upper_deps = [&](int i, auto&& f) {
-      for (int t = rp[i]; t < rp[i + 1]; ++t)
-        if (ci[t] > i) f(ci[t]);
-    };
-    pc->n_lev_lo = level_order(n, true, lower_deps, order);
-    BSP_TRY(upload(pc->order_lo, order));
-    BSP_TRY(make_tasks(pc, true, n, lower_deps));
-    pc->n_lev_up = level_order(n, false, upper_deps, order);
-    BSP_TRY(upload(pc->order_up, order));
-    BSP_TRY(make_tasks(pc, false, n, upper_deps));
-    if (wave_supported(pc->bs)) {
-      // the dependent entries of a forward (j < i) and a backward sweep
-      for (const bool fwd : {true, false}) {
-        SweepEntries ent;
-        ent.ptr.assign(n + 1, 0);
-        for (int i = 0; i < n; ++i) {
-          for (int t = rp[i]; t < rp[i + 1]; ++t)
-            if (fwd ? ci[t] < i : ci[t] > i) {
-              ent.col.push_back(ci[t]);
-              ent.blk.push_back(t);
-            }
-          ent.ptr[i + 1] = (int)ent.col.size();
-        }
-        auto& S = fwd ? pc->wv_lo : pc->wv_up;
-        S = std::make_shared<WaveSym>();
-        BSP_TRY(wave_build(n, pc->bs, fwd, ent, false, false, false, {}, 1, nullptr, nullptr, *S));
+    // the dependent entries of a forward (j < i) and a backward sweep
+    SweepPlanner sweeps;
+    SweepEntries &lo = sweeps.lo, &up = sweeps.up;
+    lo.ptr.assign(n + 1, 0);
+    up.ptr.assign(n + 1, 0);
+    for (int i = 0; i < n; ++i) {
+      for (int t = rp[i]; t < rp[i + 1]; ++t) {
+        if (ci[t] == i) continue;
+        SweepEntries& E = ci[t] < i ? lo : up;
+        E.col.push_back(ci[t]);
+        E.blk.push_back(t);
       }
+      lo.ptr[i + 1] = (int)lo.col.size();
+      up.ptr[i + 1] = (int)up.col.size();
     }
+    sweeps.in_place = true;
+    sweeps.start(n, pc->bs);
+    auto deps_of = [](const SweepEntries& E) {
+      return [&E](int i, auto&& f) {
+        for (int t = E.ptr[i]; t < E.ptr[i + 1]; ++t) f(E.col[t]);
+      };
+    };
+    pc->n_lev_lo = level_order(n, true, deps_of(lo), order);
+    BSP_TRY(upload(pc->order_lo, order));
+    BSP_TRY(make_tasks(pc, true, n, deps_of(lo)));
+    pc->n_lev_up = level_order(n, false, deps_of(up), order);
+    BSP_TRY(upload(pc->order_up, order));
+    BSP_TRY(make_tasks(pc, false, n, deps_of(up)));
+    BSP_TRY(sweeps.finish(pc->wv_lo, pc->wv_up, pc->ss_lo, pc->ss_up));
   }
   return BSP_OK;
 }
@@ -1473,8 +1455,12 @@ static int build_diag_inverse(bsp_precond_s* pc) {
 }
 
 // The factors changed: every copy of them in sweep order is stale.
-static void wave_invalidate(bsp_precond_s* pc) {
-  for (int k = 0; k < 3; ++k) pc->vv_lo[k].valid = pc->vv_up[k].valid = false;
+static void sweep_invalidate(bsp_precond_s* pc) {
+  for (int k = 0; k < 3; ++k) {
+    pc->vv_lo[k].valid = pc->vv_up[k].valid = false;
+    pc->sv_lo[k].valid = pc->sv_up[k].valid = false;
+  }
+  pc->level_ordered = false;
 }
 
 static int make_lowp_copies(bsp_precond_s* pc) {
@@ -1503,7 +1489,7 @@ static int make_lowp_copies(bsp_precond_s* pc) {
 
 int precond_build(bsp_precond_s* pc) {
   const int n = pc->n, b2 = pc->bs * pc->bs;
-  wave_invalidate(pc);
+  sweep_invalidate(pc);
   BSP_TRY(take(pc->A, pc->dinv, (size_t)std::max(n, 1) * b2));
   BSP_TRY(take(pc->A, pc->flags, std::max(n, 1)));
   BSP_TRY(take(pc->A, pc->ticket, 1));
@@ -1572,7 +1558,7 @@ static int relax_offdiag(bsp_precond_s* pc, const double* f0) {
 // from the corrected U_ii / L_ii (general inverses).
 int precond_build_learned(bsp_precond_s* pc, const double* dF) {
   const int n = pc->n, b2 = pc->bs * pc->bs;
-  wave_invalidate(pc);
+  sweep_invalidate(pc);
   BSP_TRY(take(pc->A, pc->dinv, (size_t)std::max(n, 1) * b2));
   BSP_TRY(take(pc->A, pc->flags, std::max(n, 1)));
   BSP_TRY(take(pc->A, pc->ticket, 1));
@@ -1624,28 +1610,89 @@ template <typename VT> constexpr int prec_of() {
   return std::is_same<VT, double>::value ? BSP_PREC_F64 : std::is_same<VT, float>::value ? BSP_PREC_F32 : BSP_PREC_BF16;
 }
 
-// z = M^{-1} r through the lock-step sweeps.  The values of the precision are
-// gathered on first use.
-template <typename VT>
-static int apply_wave(bsp_precond_s* pc, const double* r, double* z) {
-  bsp_handle_s* h = pc->h;
-  constexpr int prec = prec_of<VT>();
-  WaveVals& lo = pc->vv_lo[prec];
-  WaveVals& up = pc->vv_up[prec];
-  for (auto* v : {&lo, &up}) {
-    if (v->valid) continue;
-    const WaveSym& S = v == &lo ? *pc->wv_lo : *pc->wv_up;
+// The copies in sweep order that an application in precision `prec` needs, and
+// its vectors; made on first use.  Launches nothing that touches r or z.
+static int wave_ready(bsp_precond_s* pc, int prec) {
+  const bool sor = pc->kind == BSP_PC_SOR_LU || pc->kind == BSP_PC_SOR_CHOL;
+  for (const bool lower : {true, false}) {
+    const WaveSym& S = lower ? *pc->wv_lo : *pc->wv_up;
+    WaveVals& V = lower ? pc->vv_lo[prec] : pc->vv_up[prec];
+    if (sor && (lower ? pc->type < 0 : pc->type > 0)) continue;  // that direction is not swept
+    if (V.valid) continue;
     const size_t vb = wave_val_bytes(S, prec);
-    if (v->vals.n < vb) BSP_TRY(take(pc->A, v->vals, vb));
-    BSP_TRY(wave_gather(h, S, prec, pc->f_vals.get(), pc->dinv.get(), *v));
+    if (V.vals.n < vb) BSP_TRY(take(pc->A, V.vals, vb));
+    if (sor) BSP_TRY(wave_gather(pc->h, S, prec, pc->A->vals.get(), pc->dinv.get(), V, true, pc->w));
+    else BSP_TRY(wave_gather(pc->h, S, prec, pc->f_vals.get(), pc->dinv.get(), V));
   }
-  const size_t need[2] = {wave_item_values(*pc->wv_up, 1), wave_item_values(*pc->wv_lo, 1)};
-  for (int i = 0; i < 2; ++i)
+  const size_t n_lo = wave_item_values(*pc->wv_lo, 1), n_up = wave_item_values(*pc->wv_up, 1);
+  const size_t need[3] = {sor ? 0 : n_up, sor ? 0 : n_lo, sor ? std::max(n_lo, n_up) : 0};
+  for (int i = 0; i < 3; ++i)
     if (pc->s64[i].n < need[i]) BSP_TRY(take(pc->A, pc->s64[i], need[i]));
+  return BSP_OK;
+}
+static int stream_ready(bsp_precond_s* pc, int prec) {
+  for (const bool lower : {true, false}) {
+    const StreamSym& S = lower ? *pc->ss_lo : *pc->ss_up;
+    StreamVals& V = lower ? pc->sv_lo[prec] : pc->sv_up[prec];
+    if (V.valid) continue;
+    const size_t vb = stream_val_bytes(S, pc->bs, prec), db = stream_dval_bytes(S, pc->bs, prec);
+    if (V.vals.n < vb) BSP_TRY(take(pc->A, V.vals, vb));
+    if (db && V.dvals.n < db) BSP_TRY(take(pc->A, V.dvals, db));
+    BSP_TRY(stream_gather(pc->h, S, pc->bs, prec, pc->f_vals.get(), pc->dinv.get(), V));
+  }
+  return BSP_OK;
+}
+
+// Which sweeps an application with FP64 vectors runs through.  Where the copies
+// in sweep order do not fit memory the level-ordered kernels, which read the
+// factors in place, take it (until the factors change).
+enum class Path { kLevels, kWave, kStream };
+static int sweep_path(bsp_precond_s* pc, int prec, const void* r, const void* z, Path* out) {
+  *out = Path::kLevels;
+  if (pc->level_ordered) return BSP_OK;
+  const bool wave = pc->wv_lo && pc->wv_up;
+  // the streamed sweeps read vectors in 16-byte pieces
+  const bool stream = pc->ss_lo && pc->ss_up && reinterpret_cast<uintptr_t>(z) % 16 == 0 &&
+                      reinterpret_cast<uintptr_t>(r) % 16 == 0;
+  if (!wave && !stream) return BSP_OK;
+  const int st = wave ? wave_ready(pc, prec) : stream_ready(pc, prec);
+  if (st == BSP_OUT_OF_MEMORY) {
+    record_error("");
+    for (int k = 0; k < 3; ++k) {
+      pc->vv_lo[k] = WaveVals{};
+      pc->vv_up[k] = WaveVals{};
+      pc->sv_lo[k] = StreamVals{};
+      pc->sv_up[k] = StreamVals{};
+    }
+    pc->level_ordered = true;
+    // a vector that was to grow has lost its old place
+    for (auto& v : pc->s64)
+      if (v.n < (size_t)pc->n * pc->bs) BSP_TRY(take(pc->A, v, (size_t)pc->n * pc->bs));
+    return BSP_OK;
+  }
+  BSP_TRY(st);
+  *out = wave ? Path::kWave : Path::kStream;
+  return BSP_OK;
+}
+
+// z = M^{-1} r through the lock-step sweeps.
+static int apply_wave(bsp_precond_s* pc, int prec, const double* r, double* z) {
+  bsp_handle_s* h = pc->h;
   double *w = pc->s64[0].get(), *rp = pc->s64[1].get();
   BSP_TRY(wave_prepare(h, *pc->wv_lo, *pc->wv_up, r, rp, w, z));
-  BSP_TRY(wave_sweep(h, *pc->wv_lo, prec, lo, rp, w, pc->wticket.get()));
-  return wave_sweep(h, *pc->wv_up, prec, up, w, z, pc->wticket.get());
+  BSP_TRY(wave_sweep(h, *pc->wv_lo, prec, pc->vv_lo[prec], rp, w, pc->wticket.get()));
+  return wave_sweep(h, *pc->wv_up, prec, pc->vv_up[prec], w, z, pc->wticket.get());
+}
+
+// The same through the streamed sweeps.
+static int apply_stream(bsp_precond_s* pc, int prec, const double* r, double* z) {
+  bsp_handle_s* h = pc->h;
+  const int64_t nv = (int64_t)pc->n * pc->bs;
+  double* w = pc->s64[0].get();
+  BSP_TRY(fill_sentinel(h, w, nv));
+  BSP_TRY(stream_sweep(h, *pc->ss_lo, pc->bs, prec, pc->sv_lo[prec], r, w, pc->ticket.get()));
+  BSP_TRY(fill_sentinel(h, z, nv));
+  return stream_sweep(h, *pc->ss_up, pc->bs, prec, pc->sv_up[prec], w, z, pc->ticket.get());
 }
 
 // z = M^{-1} r for SOR: nu sweeps each way of x_i = c_i - sum_dep (w D_i A_ij) x_j,
@@ -1656,19 +1703,12 @@ static int apply_sor_wave(bsp_precond_s* pc, const double* r, double* z, const V
   bsp_handle_s* h = pc->h;
   const bsp_matrix_s* A = pc->A;
   constexpr int prec = prec_of<VT>();
-  const size_t need = std::max(wave_item_values(*pc->wv_lo, 1), wave_item_values(*pc->wv_up, 1));
-  if (pc->s64[2].n < need) BSP_TRY(take(pc->A, pc->s64[2], need));
   double *rp = pc->s64[2].get(), *bufs[2] = {pc->s64[0].get(), pc->s64[1].get()};
   const double* xold = nullptr;
   for (size_t s = 0; s < dirs.size(); ++s) {
     const bool fwd = dirs[s] < 0;
     const WaveSym& S = fwd ? *pc->wv_lo : *pc->wv_up;
-    WaveVals& V = fwd ? pc->vv_lo[prec] : pc->vv_up[prec];
-    if (!V.valid) {
-      const size_t vb = wave_val_bytes(S, prec);
-      if (V.vals.n < vb) BSP_TRY(take(pc->A, V.vals, vb));
-      BSP_TRY(wave_gather(h, S, prec, A->vals.get(), pc->dinv.get(), V, true, pc->w));
-    }
+    const WaveVals& V = fwd ? pc->vv_lo[prec] : pc->vv_up[prec];
     double* out = s + 1 == dirs.size() ? z : bufs[s & 1];
     BSP_TRY(wave_sor_prepare(h, S, prec, fwd, A->row_ptr.get(), A->col_idx.get(), avals, dinv, pc->w, r, xold, rp, out));
     BSP_TRY(wave_sweep(h, S, prec, V, rp, out, pc->wticket.get()));
@@ -1718,7 +1758,11 @@ static int apply_typed(bsp_precond_s* pc, const AT* r, AT* z, const VT* fvals, c
       else if (pc->type == 0) { dirs.assign(pc->nu, -1); dirs.insert(dirs.end(), pc->nu, +1); }
       else dirs.assign(pc->nu, -1);
       if constexpr (std::is_same<AT, double>::value) {
-        if (pc->wv_lo && pc->wv_up) return apply_sor_wave<VT>(pc, r, z, avals, dinv, dirs);
+        Path path;
+        BSP_TRY(sweep_path(pc, prec_of<VT>(), r, z, &path));
+        if (path == Path::kWave) return apply_sor_wave<VT>(pc, r, z, avals, dinv, dirs);
+        // an allocation may have given these another place
+        sa = pc->s64[0].get(), sb = pc->s64[1].get(), sc = pc->s64[2].get();
       }
       const AT* rhs = r;
       if (z == r) {  // in place: keep a copy of the right-hand side
@@ -1745,7 +1789,11 @@ static int apply_typed(bsp_precond_s* pc, const AT* r, AT* z, const VT* fvals, c
     case BSP_PC_ILU0:
     case BSP_PC_LEARNED_LU: {
       if constexpr (std::is_same<AT, double>::value) {
-        if (pc->wv_lo && pc->wv_up) return apply_wave<VT>(pc, r, z);
+        Path path;
+        BSP_TRY(sweep_path(pc, prec_of<VT>(), r, z, &path));
+        if (path == Path::kWave) return apply_wave(pc, prec_of<VT>(), r, z);
+        if (path == Path::kStream) return apply_stream(pc, prec_of<VT>(), r, z);
+        sa = pc->s64[0].get(), sb = pc->s64[1].get(), sc = pc->s64[2].get();
       }
       p.ptr = pc->f_ptr.get();
       p.idx = pc->f_col.get();
@@ -1772,7 +1820,11 @@ static int apply_typed(bsp_precond_s* pc, const AT* r, AT* z, const VT* fvals, c
     case BSP_PC_ICHOL0:
     case BSP_PC_LEARNED_LLT: {
       if constexpr (std::is_same<AT, double>::value) {
-        if (pc->wv_lo && pc->wv_up) return apply_wave<VT>(pc, r, z);
+        Path path;
+        BSP_TRY(sweep_path(pc, prec_of<VT>(), r, z, &path));
+        if (path == Path::kWave) return apply_wave(pc, prec_of<VT>(), r, z);
+        if (path == Path::kStream) return apply_stream(pc, prec_of<VT>(), r, z);
+        sa = pc->s64[0].get(), sb = pc->s64[1].get(), sc = pc->s64[2].get();
       }
       p.ptr = pc->f_ptr.get();
       p.idx = pc->f_col.get();
@@ -1935,7 +1987,7 @@ int precond_learned_init(bsp_precond_s* pc) {
 // (both built on the same matrix) and gets fresh diagonal inverses.
 int precond_learned_refresh(bsp_precond_s* work, const bsp_precond_s* ilu, const double* dF) {
   if (work->f_nnzb != ilu->f_nnzb || work->n != ilu->n || work->bs != ilu->bs) return BSP_INVALID;
-  wave_invalidate(work);
+  sweep_invalidate(work);
   const int b2 = work->bs * work->bs;
   const int64_t tot = work->f_nnzb * b2;
   if (tot > 0)
@@ -2076,6 +2128,8 @@ int bsp_precond_destroy(bsp_precond_t pc) {
       give(A, pc->s32[i]);
       give(A, pc->vv_lo[i].vals);
       give(A, pc->vv_up[i].vals);
+      give(A, pc->sv_lo[i].vals); give(A, pc->sv_lo[i].dvals);
+      give(A, pc->sv_up[i].vals); give(A, pc->sv_up[i].dvals);
     }
   }
   delete pc;

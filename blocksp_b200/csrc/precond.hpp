@@ -2,6 +2,7 @@
 // single-system, batched and learned solvers).
 #pragma once
 #include "internal.hpp"
+#include "sweep_stream.hpp"
 #include "sweep_wave.hpp"
 
 namespace bsp {
@@ -75,6 +76,11 @@ struct bsp_precond_s {
   std::shared_ptr<bsp::WaveSym> wv_lo, wv_up;
   bsp::WaveVals vv_lo[3], vv_up[3];
   bsp::DevBuf<unsigned> wticket;  // 0 between sweeps (every sweep resets it)
+  // the same for the streamed sweeps, which take 8 x 8 and 16 x 16 blocks where
+  // the lock-step ones are slower (sweep_cost.h; at most one of the two is laid out)
+  std::shared_ptr<bsp::StreamSym> ss_lo, ss_up;
+  bsp::StreamVals sv_lo[3], sv_up[3];
+  bool level_ordered = false;  // neither's copies fitted memory
   // elimination plan of the factorisation (shared with the matrix's cache)
   std::shared_ptr<bsp::FactorPlan> plan;
 };

@@ -10,30 +10,6 @@ namespace bsp {
 
 int grid_for(const bsp_handle_s* h, int64_t n, int threads);
 
-#define BSP_WAVE_SIZES(X) X(1) X(2) X(3) X(4) X(5) X(6) X(8) X(16)
-
-bool wave_supported(int bs) {
-  switch (bs) {
-#define BSP_WAVE_CASE(B) case B:
-    BSP_WAVE_SIZES(BSP_WAVE_CASE)
-#undef BSP_WAVE_CASE
-    return true;
-    default: return false;
-  }
-}
-
-WaveShape wave_shape(int bs, int nrhs) {
-  WaveShape s;
-  switch (bs) {
-#define BSP_WAVE_CASE(B) \
-  case B: s = nrhs == 1 ? wave_shape_of<B, 1>() : wave_shape_of<B, 2>(); break;
-    BSP_WAVE_SIZES(BSP_WAVE_CASE)
-#undef BSP_WAVE_CASE
-    default: break;
-  }
-  return s;
-}
-
 // ------------------------------------------------------------------ values
 // Stored block b: minus w times factor block blk_src[b] (transposed when
 // trans), or what the negative codes of wave_plan.h say.
@@ -255,14 +231,9 @@ template <typename T, typename H> static int upload_as(DevBuf<T>& d, const std::
   return BSP_OK;
 }
 
-int wave_build(int n, int bs, bool ascending, const SweepEntries& ent, bool trans_blocks, bool has_d, bool trans_d,
-               const std::vector<int>& group_beg, int nrhs, const std::vector<int>* row_item,
-               std::vector<int>* item_of, WaveSym& S) {
-  WavePlan P;
-  if (!wave_plan(n, ascending, wave_shape(bs, nrhs), has_d, ent, group_beg, P)) {
-    record_error("triangular sweep: the dependencies are not triangular, or the stream is too long");
-    return BSP_INVALID;
-  }
+int wave_upload(WavePlan&& P, int bs, bool trans_blocks, bool has_d, bool trans_d, const std::vector<int>* row_item,
+                std::vector<int>* item_of, WaveSym& S) {
+  const int n = P.n;
   std::vector<int> items(n, 0);
   for (size_t i = 0; i < P.item_row.size(); ++i)
     if (P.item_row[i] >= 0) items[P.item_row[i]] = (int)i;

@@ -52,44 +52,6 @@
 
 namespace bsp {
 
-constexpr int kWaveWarps = 8;   // compute warps of a set
-constexpr int kSlots = 8;       // steps staged ahead
-constexpr int kRing = 8;        // steps whose results stay in shared memory
-
-// Lanes and CTA shape of a block size.  Sizes 1, 2, 4, 8, 16: row-major
-// blocks, lane l of a block's G holds pieces q * G + l of V values, those of PR
-// block rows.  Others (3, 5, 6): column-major blocks, lane r holds block row r.
-// A step begins with the operand reads of its 8 warps all at once, and the
-// lanes that hold different rows of a block read the same operands again, so a
-// block is spread over as few lanes as its registers allow.  8 x 8 over 16 lanes, two rows each, two items
-// side by side, against a warp an item and two items in turn: 64^3 application
-// 321 -> 300 us, 160 x 160 (IChol0) 298 -> 267, batched sweeps with 4
-// right-hand sides 258 -> 175 us.  16 x 16 in one warp, four rows a lane in
-// FP64, against two warps: 48^3 363 -> 351 us, 80 x 80 (IChol0) 1159 -> 607.  With
-// several right-hand sides the registers do not suffice for that.
-template <int BS, int R = 1> struct WaveDim {
-  static constexpr bool kChunk = (BS & (BS - 1)) == 0;
-  static constexpr int G = BS == 1 ? 1 : BS == 2 ? 2 : BS == 3 ? 4 : BS < 8 ? 8 : BS == 8 ? 16 : 32;  // lanes of a warp per item
-  static constexpr int WPI = BS == 16 && R > 1 ? 2 : 1;                               // warps per item
-  static constexpr int IPW = 32 / G;                                                   // items side by side in a warp
-  static constexpr bool kItemMajor = BS >= 4;                                          // order of a step's blocks
-  static constexpr int W = kWaveWarps * IPW / WPI;
-  static constexpr int ECAP = W >= 128 ? 64 : W >= 64 ? 32 : W >= 16 ? 16 : 8;
-};
-// External rows of a step with R right-hand sides: with more than one, what the
-// tile of a 3D grid needs (the fetch warps hold them in registers).
-template <int BS, int R> constexpr int wave_ecap() { return R == 1 ? WaveDim<BS>::ECAP : BS == 4 ? 12 : 8; }
-
-template <int BS, int R> inline WaveShape wave_shape_of() {
-  WaveShape s;
-  s.W = WaveDim<BS, R>::W;
-  s.ecap = wave_ecap<BS, R>();
-  s.ring = kRing;
-  s.slots = kSlots;
-  s.item_major = WaveDim<BS>::kItemMajor;
-  return s;
-}
-
 template <int BS, typename VT, int R> struct WaveMap : WaveDim<BS, R> {
   using D = WaveDim<BS, R>;
   static constexpr int V = !D::kChunk ? BS : BS == 1 ? 1 : BS < 16 ? 2 : sizeof(VT) == 8 ? 2 : 4;
@@ -118,10 +80,7 @@ template <int BS, typename VT, bool HAS_D, int NE, int R> struct WaveCfg {
   static constexpr int OFF_HDR = OFF_REC + kSlots * M::W * 16;  // {first item, items} of every staged step
   static constexpr int OFF_BAR = OFF_HDR + kSlots * 8;
   static constexpr int kSmem = OFF_BAR + 3 * kSlots * 8;
-  // three turns of polls in flight keep up with the short steps of small blocks
-  // (24 x 20 rows of 2 x 2 blocks 42.7 -> 39.4 us, 40 x 36 x 44 of 4 x 4 133 -> 125);
-  // larger ones need the registers (64^3 of 8 x 8: 321 -> 327 us with three)
-  static constexpr int kFetchWarps = R == 1 && BS <= 4 ? 3 : 2;
+  static constexpr int kFetchWarps = M::kFetchWarps;
   static constexpr int kThreads = (2 * kWaveWarps + 2 + kFetchWarps) * 32;
   static_assert(kSmem <= 226 * 1024, "a CTA's vector rows do not fit shared memory");
 };

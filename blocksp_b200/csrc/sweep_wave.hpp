@@ -15,7 +15,7 @@
 #include <memory>
 #include <vector>
 #include "internal.hpp"
-#include "wave_plan.h"
+#include "wave_shape.h"
 
 namespace bsp {
 
@@ -33,19 +33,12 @@ struct WaveSym {
   DevBuf<int64_t> blk_src;
 };
 
-// Block sizes the lock-step kernel takes (FP64 vectors).
-bool wave_supported(int bs);
-WaveShape wave_shape(int bs, int nrhs);
-
-// Plans and uploads the sweep over n rows; ascending: forward (dependencies
-// j < i), else backward (j > i).  group_beg: see wave_plan; nrhs: right-hand
-// sides of a row (the plans for 2 and 4 are the same).  A sweep reads its
-// right-hand side in item order; one that is followed by another writes its
-// result in that one's item order: row_item is, per row, the item that reads
-// it (null: natural order), and item_of receives that of this sweep.
-int wave_build(int n, int bs, bool ascending, const SweepEntries& ent, bool trans_blocks, bool has_d, bool trans_d,
-               const std::vector<int>& group_beg, int nrhs, const std::vector<int>* row_item,
-               std::vector<int>* item_of, WaveSym& S);
+// Uploads a plan (wave_plan.h).  A sweep reads its right-hand side in item
+// order; one that is followed by another writes its result in that one's item
+// order: row_item is, per row, the item that reads it (null: natural order),
+// and item_of receives that of this sweep.
+int wave_upload(WavePlan&& P, int bs, bool trans_blocks, bool has_d, bool trans_d, const std::vector<int>* row_item,
+                std::vector<int>* item_of, WaveSym& S);
 // Values of a vector of one value set per item (1 right-hand side).
 size_t wave_item_values(const WaveSym& S, int nrhs);
 

@@ -28,8 +28,11 @@
 #pragma once
 #include <algorithm>
 #include <cstdint>
+#include <functional>
+#include <limits>
 #include <map>
 #include <numeric>
+#include <queue>
 #include <vector>
 
 namespace bsp {
@@ -50,6 +53,8 @@ struct WaveShape {
   int ring = 0;   // steps whose results stay in shared memory
   int slots = 0;  // steps whose right-hand sides and external rows are staged
   bool item_major = false;  // order of a step's blocks, see WaveStep
+  int fetch = 2;            // warps that bring in external rows, a step each in turn
+  double step_us = 0.3;     // time of a step that waits for nothing
   // vector rows in shared memory, in this order
   int n_rows() const { return ring * W + 1 + slots * (W + ecap); }
   int result(int step, int item) const { return step % ring * W + item; }
@@ -84,6 +89,8 @@ constexpr int64_t kWaveOne = -3;   // the identity (D of a continued row)
 struct WavePlan {
   int n = 0, n_super = 0, n_levels = 0;
   int ne = 0;                    // entries of an item
+  bool over_limit = false;       // given up: its estimate passed the caller's limit
+  double est_us = 0.0;           // estimated time of the sweep, see WaveClock
   std::vector<int> super_step;   // n_super + 1
   std::vector<int> super_group;  // group of each super-task
   std::vector<WaveStep> step;    // all steps + 1
@@ -133,7 +140,7 @@ inline bool group_rows(int r0, int r1, bool ascending, const WaveShape& S, const
   const int nc = (int)first.size();
   // distinct predecessor chains of every chain, and their strides
   std::vector<std::vector<int>> cdeps(nc);
-  std::map<int, int> stride_count;
+  std::vector<int> stride_count(nc + 1, 0);
   for (int c = 0; c < nc; ++c) {
     auto& dc = cdeps[c];
     for (int k = 0; k < clen[c]; ++k) {
@@ -183,10 +190,10 @@ inline bool group_rows(int r0, int r1, bool ascending, const WaveShape& S, const
     return (int)queue.size() == nsup;
   };
   int dom = 0, dom_n = 0;
-  for (auto& kv : stride_count)
-    if (kv.second > dom_n) {
-      dom = kv.first;
-      dom_n = kv.second;
+  for (int d = 2; d <= nc; ++d)
+    if (stride_count[d] > dom_n) {
+      dom = d;
+      dom_n = stride_count[d];
     }
   int wz = 1;
   while (wz * wz * 4 <= S.W) wz *= 2;  // 16 -> 4 x 4, 8 -> 4 x 2, 64 -> 8 x 8
@@ -220,14 +227,58 @@ inline bool group_rows(int r0, int r1, bool ascending, const WaveShape& S, const
   return true;
 }
 
+// Estimated time of a sweep: the CTAs take super-tasks in ticket order; a step
+// starts when the one before is over and its external rows are there, which a
+// fetch warp reads in about kFetchUs when they are published already and
+// kHopUs after they are published otherwise.  Fitted to measured applications
+// (step times per block size in wave_shape.h): within 20 % on most of 23
+// patterns and 8 block sizes, grids and random orders alike; grids bound by
+// bandwidth are up to 40 % slower than it says.
+constexpr int kClockCtas = 148;
+constexpr double kStartUs = 1.5, kHopUs = 1.2, kFetchUs = 0.8;
+class WaveClock {
+  std::vector<double> done_, fetch_;
+  std::priority_queue<double, std::vector<double>, std::greater<double>> cta_;
+
+ public:
+  double end = 0.0;
+  WaveClock(int n, const WaveShape& S) : done_(n, 0.0), fetch_(S.fetch, 0.0) {
+    for (int i = 0; i < kClockCtas; ++i) cta_.push(0.0);
+  }
+  // the last super-task of P, its steps from `first` on
+  void super_task(const WavePlan& P, const WaveShape& S, size_t first) {
+    double now = cta_.top() + kStartUs;
+    cta_.pop();
+    std::fill(fetch_.begin(), fetch_.end(), now);
+    for (size_t s = first; s < P.step.size(); ++s) {
+      const bool last = s + 1 == P.step.size();
+      const size_t i1 = last ? P.rec.size() : P.step[s + 1].item0, e1 = last ? P.ext_row.size() : P.step[s + 1].ext0;
+      if ((size_t)P.step[s].ext0 < e1) {
+        double there = 0.0;
+        for (size_t e = P.step[s].ext0; e < e1; ++e) there = std::max(there, done_[P.ext_row[e]]);
+        double& f = fetch_[(s - first) % fetch_.size()];
+        f = std::max(f + kFetchUs, there + kHopUs);
+        now = std::max(now, f);
+      }
+      now += S.step_us;
+      for (size_t i = P.step[s].item0; i < i1; ++i)
+        if (P.rec[i].row >= 0) done_[P.rec[i].row] = now;
+    }
+    cta_.push(now);
+    end = std::max(end, now);
+  }
+};
+
 }  // namespace wave_detail
 
 // The layout of a sweep over n rows; ascending: forward (dependencies j < i),
 // else backward.  has_d: rows carry a D block.  group_beg: first row of every
 // independent group, then n (empty: one group).  False when the dependencies
-// are not triangular or the stream is too long.
+// are not triangular, the stream is too long, or the sweep would take more than
+// limit_us (over_limit; planning stops there).
 inline bool wave_plan(int n, bool ascending, const WaveShape& S, bool has_d, const SweepEntries& E,
-                      const std::vector<int>& group_beg, WavePlan& P) {
+                      const std::vector<int>& group_beg, WavePlan& P,
+                      double limit_us = std::numeric_limits<double>::infinity()) {
   using namespace wave_detail;
   P = WavePlan{};
   P.n = n;
@@ -263,11 +314,14 @@ inline bool wave_plan(int n, bool ascending, const WaveShape& S, bool has_d, con
   std::vector<std::vector<int>> ext;
   std::vector<std::pair<int, int>> ord, seg;  // (step of the dependency or -1, entry); (first, count)
   std::vector<int> at;
+  WaveClock clock(n, S);
   for (int sid : order) {
     const Sup& sp = sups[sid];
     P.n_levels = std::max(P.n_levels, sp.level + 1);
     size_t used = 0;  // steps of this super-task: their lists keep what they held room for
-    size_t hint = 0;  // steps before it are full
+    // steps before room[k] are full, or have no room for k external rows (both
+    // only fill up): without it a row of external rows passes over every step
+    size_t room[kMaxEnt + 1] = {};
     for (int r : sp.rows) {
       ord.clear();
       int lo = 0;
@@ -294,7 +348,11 @@ inline bool wave_plan(int n, bool ascending, const WaveShape& S, bool has_d, con
         }
         return need == 0 || have + need <= S.ecap;
       };
-      while (hint < used && (int)st[hint].size() >= S.W) ++hint;
+      // external rows of the first segment wherever it goes
+      int far = 0;
+      while (far < seg[0].second && ord[far].first < 0) ++far;
+      size_t& hint = room[far];
+      while (hint < used && ((int)st[hint].size() >= S.W || (far > 0 && (int)ext[hint].size() + far > S.ecap))) ++hint;
       at.assign(ns, 0);
       for (int base = std::max({lo - ns + 1, 0, (int)hint});; ++base) {
         bool good = true;
@@ -347,6 +405,7 @@ inline bool wave_plan(int n, bool ascending, const WaveShape& S, bool has_d, con
       r_item[r] = prev_item;
     }
     // flatten
+    const size_t first_step = P.step.size();
     for (size_t s = 0; s < used; ++s) {
       P.step.push_back({(int32_t)P.rec.size(), (int32_t)P.ext_row.size()});
       for (const Item& it : st[s]) {
@@ -370,9 +429,16 @@ inline bool wave_plan(int n, bool ascending, const WaveShape& S, bool has_d, con
     }
     P.super_step.push_back((int)P.step.size());
     P.super_group.push_back(sp.group);
+    if (P.blk_src.size() >= (size_t)INT32_MAX || P.ext_row.size() >= (size_t)INT32_MAX) return false;
+    clock.super_task(P, S, first_step);
+    P.est_us = clock.end;
+    if (clock.end > limit_us) {
+      P.over_limit = true;
+      return false;
+    }
   }
   P.step.push_back({(int32_t)P.rec.size(), (int32_t)P.ext_row.size()});
-  return P.blk_src.size() < (size_t)INT32_MAX && P.ext_row.size() < (size_t)INT32_MAX && S.n_rows() <= 0xffff;
+  return S.n_rows() <= 0xffff;
 }
 
 }  // namespace bsp
