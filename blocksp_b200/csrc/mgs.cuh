@@ -10,7 +10,12 @@
 // one step, and the coefficients follow as modified Gram-Schmidt gives them,
 //   h_k = <q_k, v> - sum_{i<k} <q_k, q_i> h_i
 // (the triangular form of the same recurrence: h_k is the product with v after
-// the updates by q_i, i < k), before v takes the B updates in order.  So a
+// the updates by q_i, i < k), before v takes the B updates in order.  In exact
+// arithmetic that is modified Gram-Schmidt; in rounding h_k carries eps ||v|| of
+// the block's start where that carries eps ||v|| after the updates before it, up
+// to B vectors at a time.  Both lose orthogonality like eps times the condition
+// of the columns, and histories of nearly dependent columns are off 80-bit
+// arithmetic by as much as plain modified Gram-Schmidt is.  So a
 // column costs a grid barrier per B vectors instead of one per vector, and every
 // basis vector is still read once.  Steps are separated by a bounded grid
 // barrier; every CTA sums the per-CTA partials in index order, so H is
