@@ -16,6 +16,8 @@
 //     the block-diagonal of the per-system factors, so the factorisation runs
 //     once over the whole group, and the lock-step sweeps (sweep_wave.cuh) run
 //     the super-tasks of every system in one launch, a system's own plan each;
+//     a group whose rows are in an order that does not suit them is swept row by
+//     row (batch_sweep.cuh; sweep_cost.h states the rule);
 //   * right-hand sides are interleaved per block row (the solArray<T,bs,R>
 //     layout), so each matrix / factor block is read once for all R of them;
 //   * per-pair scalars come from segmented reductions over fixed tiles of a few
@@ -28,17 +30,19 @@
 //     of the same iteration graph is kept as the alternative mode);
 //   * converged systems drop out: every tile, task and reduction of a system
 //     whose pairs are all finished is skipped;
-//   * launch shapes (threads per CTA and CTAs per SM of the tile kernels) are
-//     chosen per group by timing the candidates on the group's own data the
-//     first time it is solved (an autotuner).
+//   * launch shapes (threads per CTA and CTAs per SM of the tile kernels, CTAs
+//     per SM of the level-ordered sweeps) are chosen per group by timing the
+//     candidates on the group's own data the first time it is solved (an
+//     autotuner).
 #include <algorithm>
 #include <chrono>
 #include <cstring>
 #include <functional>
 #include <numeric>
 #include <vector>
+#include "batch_sweep.cuh"
 #include "precond.hpp"
-#include "sentinel.cuh"
+#include "sweep_plan.hpp"
 
 namespace bsp {
 
@@ -76,9 +80,12 @@ struct BGroupP {
   const double* vals;
   double *x, *r, *z, *w, *p, *q, *part0, *part1;
   double* rp;               // r in the forward sweep's item order
-  const int *item_lo, *item_up;  // per row: its item of the forward / backward sweep
+  // per row: its item of the forward / backward sweep (null: the level-ordered
+  // sweeps, which read r and write w row by row)
+  const int *item_lo, *item_up;
   BState* st;
   int* sys_active;
+  unsigned* tickets;        // [0] forward sweep, [1] backward sweep
   double* hist;
   int hist_cap;
   const BOpts* opts;
@@ -220,6 +227,16 @@ template <int BS, int R> __device__ __forceinline__ int64_t item_place(const int
   const int64_t row = e / (R * BS);
   return (int64_t)__ldg(item + row) * (R * BS) + (e - row * (R * BS));
 }
+// Element e of the residual is rv: the sweeps' copy of it and their sentinels.
+template <int BS, int R> __device__ __forceinline__ void start_sweeps(const BGroupP& g, int64_t e, double rv) {
+  int64_t we = e;
+  if (g.item_lo) {
+    g.rp[item_place<BS, R>(g.item_lo, e)] = rv;
+    we = item_place<BS, R>(g.item_up, e);
+  }
+  reinterpret_cast<unsigned long long*>(g.w)[we] = kSentinel64;
+  reinterpret_cast<unsigned long long*>(g.z)[e] = kSentinel64;
+}
 
 // x += alpha p, r -= alpha q for running pairs; part1 = r . r; r goes to the
 // forward sweep's item order too, and the sweep outputs w (in the backward
@@ -249,9 +266,7 @@ __global__ void __launch_bounds__(kBatchMaxThreads) k_bt_update(const BGroupP g)
       const double sq = rv * rv;
 #pragma unroll
       for (int k = 0; k < R; ++k) acc[k] += (k == rhs) ? sq : 0.0;
-      g.rp[item_place<BS, R>(g.item_lo, e)] = rv;
-      reinterpret_cast<unsigned long long*>(g.w)[item_place<BS, R>(g.item_up, e)] = kSentinel64;
-      reinterpret_cast<unsigned long long*>(g.z)[e] = kSentinel64;
+      start_sweeps<BS, R>(g, e, rv);
     }
     store_partials<R>(g.part1, t, acc);
   }
@@ -308,9 +323,7 @@ __global__ void __launch_bounds__(kBatchMaxThreads) k_bt_init(const BGroupP g) {
     BT_FOR_ELEMS(e, rhs, r0, r1) {
       (void)rhs;
       g.x[e] = 0.0;
-      g.rp[item_place<BS, R>(g.item_lo, e)] = g.r[e];
-      reinterpret_cast<unsigned long long*>(g.w)[item_place<BS, R>(g.item_up, e)] = kSentinel64;
-      reinterpret_cast<unsigned long long*>(g.z)[e] = kSentinel64;
+      start_sweeps<BS, R>(g, e, g.r[e]);
     }
   }
 }
@@ -350,6 +363,7 @@ template <int R, int MODE>
 __global__ void __launch_bounds__(kFinThreads) k_bt_fin(const BGroupP g) {
   __shared__ double part[2][kFinThreads / 32][R];
   const int s = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (MODE == FIN_RES && s == 0 && threadIdx.x < 2) g.tickets[threadIdx.x] = 0u;
   if (MODE != FIN_INIT && !g.sys_active[s]) return;
   const int t0 = g.sys_tile[s], t1 = g.sys_tile[s + 1];
   const double* src = (MODE == FIN_RES) ? g.part1 : g.part0;
@@ -473,7 +487,7 @@ namespace {
 
 struct TuneCfg {
   int threads = 256, ctas_per_sm = 2;   // tile kernels
-  int sweep_ctas_per_sm = 1;            // the sweeps run one CTA per SM
+  int sweep_ctas_per_sm = 1;            // lock-step sweeps: one CTA per SM; others: 0 is the occupancy maximum
 };
 
 struct BatchGroup {
@@ -483,11 +497,13 @@ struct BatchGroup {
   bsp_matrix_t A = nullptr;
   bsp_precond_t pc = nullptr;
   int n_tiles = 0;
-  DevBuf<int> tile_sys, tile_row, sys_tile;
+  DevBuf<int> tile_sys, tile_row, sys_tile, task_sys_lo, task_sys_up;
   DevBuf<int64_t> sys_row, user_off;
   // per-solve state for R right-hand sides
   int R = 0, hist_cap = 0;
-  // the two sweeps for this R (super-tasks stay inside a system)
+  // the two sweeps for this R: lock-step (super-tasks stay inside a system), or
+  // by levels, which read the preconditioner's factor
+  bool by_levels = false;
   WaveSym lo, up;
   WaveVals v_lo, v_up;
   DevBuf<double> x, r, rp, z, w, p, q, part0, part1, hist;
@@ -560,12 +576,51 @@ BGroupP view(bsp_batch_s* B, BatchGroup& g) {
   v.st = g.st.get();
   v.sys_active = g.sys_active.get();
   v.rp = g.rp.get();
-  v.item_lo = g.lo.item_of.get();
-  v.item_up = g.up.item_of.get();
+  v.item_lo = g.by_levels ? nullptr : g.lo.item_of.get();
+  v.item_up = g.by_levels ? nullptr : g.up.item_of.get();
+  v.tickets = g.tickets.get();
   v.hist = g.hist_cap > 0 ? g.hist.get() : nullptr;
   v.hist_cap = g.hist_cap;
   v.opts = B->opts.get();
   return v;
+}
+
+BSweepP sweep_params(bsp_batch_s* B, BatchGroup& g, bool fwd) {
+  bsp_precond_s* pc = g.pc;
+  BSweepP p{};
+  p.sys_active = g.sys_active.get();
+  p.dinv = pc->dinv.get();
+  p.vals = pc->f_vals.get();
+  p.st = B->h->ws.status.get();
+  p.spin_limit = B->h->spin_limit;
+  if (fwd) {
+    p.n_tasks = pc->n_task_lo;
+    p.task_row = pc->task_lo_row.get();
+    p.task_len = pc->task_lo_len.get();
+    p.task_sys = g.task_sys_lo.get();
+    p.task_dir = 1;
+    p.ptr = pc->f_ptr.get();
+    p.idx = pc->f_col.get();
+    p.diag = pc->f_diag.get();
+    p.blk = nullptr;
+    p.rhs = g.r.get();
+    p.x = g.w.get();
+    p.ticket = g.tickets.get();
+  } else {
+    p.n_tasks = pc->n_task_up;
+    p.task_row = pc->task_up_row.get();
+    p.task_len = pc->task_up_len.get();
+    p.task_sys = g.task_sys_up.get();
+    p.task_dir = -1;
+    p.ptr = pc->t_ptr.get();
+    p.idx = pc->t_row.get();
+    p.blk = pc->t_blk.get();
+    p.diag = nullptr;
+    p.rhs = g.w.get();
+    p.x = g.z.get();
+    p.ticket = g.tickets.get() + 1;
+  }
+  return p;
 }
 
 // Kernel set of one (block size, R) instantiation.
@@ -580,13 +635,15 @@ struct Kernels {
   void (*fin_alpha)(const BGroupP);
   void (*fin_res)(const BGroupP);
   void (*fin_beta)(const BGroupP);
+  void (*sweep_fwd)(const BSweepP);
+  void (*sweep_bwd)(const BSweepP);
 };
 
 template <int BS, int R> Kernels kernels_t() {
   return Kernels{k_bt_spmv<BS, R>,        k_bt_update<BS, R>,      k_bt_dot_rz<BS, R>,
                  k_bt_pupd<BS, R>,        k_bt_init<BS, R>,        k_bt_init_dots<BS, R>,
                  k_bt_fin<R, FIN_INIT>,   k_bt_fin<R, FIN_ALPHA>,  k_bt_fin<R, FIN_RES>,
-                 k_bt_fin<R, FIN_BETA>};
+                 k_bt_fin<R, FIN_BETA>,   k_bt_sweep<BS, R, false>, k_bt_sweep<BS, R, true>};
 }
 
 template <int BS> bool kernels_r(int R, Kernels& k) {
@@ -607,8 +664,24 @@ bool kernels_for(int bs, int R, Kernels& k) {
   }
 }
 
+int sweep_grid(bsp_batch_s* B, BatchGroup& g, void (*kern)(const BSweepP)) {
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBSweepThreads, 0) != cudaSuccess || per_sm < 1) {
+    cudaGetLastError();
+    per_sm = 1;
+  }
+  if (g.tune.sweep_ctas_per_sm > 0) per_sm = std::min(per_sm, g.tune.sweep_ctas_per_sm);
+  return grid_of(B, per_sm);
+}
+
 // w = L^-1 r, z = L^-T w for every active system.
-int enqueue_sweeps(bsp_batch_s* B, BatchGroup& g, cudaStream_t s) {
+int enqueue_sweeps(bsp_batch_s* B, BatchGroup& g, const Kernels& k, cudaStream_t s) {
+  if (g.by_levels) {
+    k.sweep_fwd<<<sweep_grid(B, g, k.sweep_fwd), kBSweepThreads, 0, s>>>(sweep_params(B, g, true));
+    k.sweep_bwd<<<sweep_grid(B, g, k.sweep_bwd), kBSweepThreads, 0, s>>>(sweep_params(B, g, false));
+    BSP_CUDA_TRY(cudaPeekAtLastError());
+    return BSP_OK;
+  }
   unsigned* tk = g.tickets.get();
   BSP_TRY(wave_sweep_multi(B->h, g.lo, g.v_lo, g.R, g.rp.get(), g.w.get(), tk, g.sys_active.get(), s));
   return wave_sweep_multi(B->h, g.up, g.v_up, g.R, g.w.get(), g.z.get(), tk + 1, g.sys_active.get(), s);
@@ -622,7 +695,8 @@ int enqueue_group(bsp_batch_s* B, BatchGroup& g, const Kernels& k, cudaStream_t 
   if (init) {
     k.init<<<tg, tt, 0, s>>>(v);
     cudaMemsetAsync(g.sys_active.get(), 1, g.n_sys() * sizeof(int), s);
-    BSP_TRY(enqueue_sweeps(B, g, s));
+    cudaMemsetAsync(g.tickets.get(), 0, 2 * sizeof(unsigned), s);
+    BSP_TRY(enqueue_sweeps(B, g, k, s));
     k.init_dots<<<tg, tt, 0, s>>>(v);
     k.fin_init<<<fin_grid, kFinThreads, 0, s>>>(v);
     n += 5;
@@ -631,8 +705,8 @@ int enqueue_group(bsp_batch_s* B, BatchGroup& g, const Kernels& k, cudaStream_t 
   k.spmv<<<tg, tt, 0, s>>>(v);
   k.fin_alpha<<<fin_grid, kFinThreads, 0, s>>>(v);
   k.update<<<tg, tt, 0, s>>>(v);
-  k.fin_res<<<fin_grid, kFinThreads, 0, s>>>(v);
-  BSP_TRY(enqueue_sweeps(B, g, s));
+  k.fin_res<<<fin_grid, kFinThreads, 0, s>>>(v);  // also zeroes the sweep tickets
+  BSP_TRY(enqueue_sweeps(B, g, k, s));
   k.dot_rz<<<tg, tt, 0, s>>>(v);
   k.fin_beta<<<fin_grid, kFinThreads, 0, s>>>(v);
   k.pupd<<<tg, tt, 0, s>>>(v);
@@ -672,8 +746,9 @@ int enqueue_phase(bsp_batch_s* B, const std::vector<Kernels>& ks, cudaStream_t s
 }
 
 // The factor's sweeps over the group's systems for R right-hand sides: plans,
-// values, and the items of every row.  The preconditioner sorts the lower
-// blocks of a row by column and stores them row by row, the diagonal last.
+// values, and the items of every row, or none where the rows go by levels.  The
+// preconditioner sorts the lower blocks of a row by column and stores them row
+// by row, the diagonal last.
 int build_sweeps(bsp_batch_s* B, BatchGroup& g, int R) {
   const int n = (int)g.n_rows();
   const auto& rp = g.A->h_row_ptr;
@@ -708,15 +783,27 @@ int build_sweeps(bsp_batch_s* B, BatchGroup& g, int R) {
       up.col[p] = i;
       up.blk[p] = lo.blk[t];
     }
-  std::vector<int> beg(g.row_off.begin(), g.row_off.end()), iu;
+  const std::vector<int> beg(g.row_off.begin(), g.row_off.end());
   g.lo = WaveSym{};
   g.up = WaveSym{};
+  g.v_lo = WaveVals{};
+  g.v_up = WaveVals{};
   const WaveShape S = wave_shape(g.bs, R);
   WavePlan p_lo, p_up;
-  if (!wave_plan(n, false, S, true, up, beg, p_up) || !wave_plan(n, true, S, true, lo, beg, p_lo)) {
-    record_error("batched sweeps: the layout is too long");
-    return BSP_INVALID;
-  }
+  bool ok[2];
+  double cost[2];
+  const bool beside = n >= kThreadRows;
+  both(beside, [&] { cost[0] = batch_sweep_cost_us(g.bs, R, n, true, lo); },
+       [&] { cost[1] = batch_sweep_cost_us(g.bs, R, n, false, up); });
+  const double limit = kWaveShare * (cost[0] + cost[1]);
+  both(beside, [&] { ok[0] = wave_plan(n, true, S, true, lo, beg, p_lo, limit); },
+       [&] { ok[1] = wave_plan(n, false, S, true, up, beg, p_up, limit); });
+  const bool was = g.by_levels;
+  g.by_levels = !(ok[0] && ok[1] && p_lo.est_us + p_up.est_us <= limit);
+  if (was != g.by_levels) g.tuned = false;
+  g.tune.sweep_ctas_per_sm = g.by_levels ? 0 : 1;
+  if (g.by_levels) return BSP_OK;
+  std::vector<int> iu;
   BSP_TRY(wave_upload(std::move(p_up), g.bs, true, true, true, nullptr, &iu, g.up));
   BSP_TRY(wave_upload(std::move(p_lo), g.bs, false, true, false, &iu, nullptr, g.lo));
   BSP_TRY(wave_gather(B->h, g.lo, BSP_PREC_F64, g.pc->f_vals.get(), g.pc->dinv.get(), g.v_lo));
@@ -732,9 +819,9 @@ int alloc_state(bsp_batch_s* B, BatchGroup& g, int R, int hist_cap) {
       BSP_TRY(v->alloc(nv));
       BSP_CUDA_TRY(cudaMemset(v->get(), 0, nv * sizeof(double)));
     }
-    BSP_TRY(g.rp.alloc(wave_item_values(g.lo, R)));
-    BSP_CUDA_TRY(cudaMemset(g.rp.get(), 0, g.rp.n * sizeof(double)));
-    BSP_TRY(g.w.alloc(wave_item_values(g.up, R)));
+    BSP_TRY(g.rp.alloc(g.by_levels ? 0 : wave_item_values(g.lo, R)));
+    if (g.rp.n) BSP_CUDA_TRY(cudaMemset(g.rp.get(), 0, g.rp.n * sizeof(double)));
+    BSP_TRY(g.w.alloc(g.by_levels ? nv : wave_item_values(g.up, R)));
     BSP_CUDA_TRY(cudaMemset(g.w.get(), 0, g.w.n * sizeof(double)));
     BSP_TRY(g.part0.alloc((size_t)g.n_tiles * R));
     BSP_TRY(g.part1.alloc((size_t)g.n_tiles * R));
@@ -774,8 +861,8 @@ float time_ms(cudaStream_t s, const std::function<void()>& f, int reps) {
 }
 
 // Autotuner: time each candidate launch shape on the group's own data.  The
-// candidates compute identical results (reductions are per fixed tile), so only
-// speed differs.
+// candidates compute identical results (reductions are per fixed tile, a row's
+// sweep does not depend on scheduling), so only speed differs.
 int autotune(bsp_batch_s* B, BatchGroup& g, const Kernels& k) {
   cudaStream_t s = B->cap;
   BSP_CUDA_TRY(cudaMemsetAsync(g.sys_active.get(), 1, g.n_sys() * sizeof(int), s));
@@ -800,6 +887,30 @@ int autotune(bsp_batch_s* B, BatchGroup& g, const Kernels& k) {
   }
   g.tune.threads = bestc.threads;
   g.tune.ctas_per_sm = bestc.ctas_per_sm;
+  // level-ordered sweeps: CTAs per SM of the persistent grid
+  if (g.by_levels) {
+    int occ = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k.sweep_fwd, kBSweepThreads, 0);
+    occ = std::max(occ, 1);
+    const BSweepP fw = sweep_params(B, g, true);
+    best = 1e30f;
+    int best_sw = occ;
+    for (int cps : {1, 2, 4, 8}) {
+      if (cps > occ) continue;
+      const int grid = grid_of(B, cps);
+      const float ms = time_ms(s, [&] {
+        k.init<<<grid_of(B, g.tune.ctas_per_sm), g.tune.threads, 0, s>>>(v);
+        cudaMemsetAsync(g.tickets.get(), 0, sizeof(unsigned), s);
+        k.sweep_fwd<<<grid, kBSweepThreads, 0, s>>>(fw);
+      }, 3);
+      bsp::count_launch_add(8);
+      if (ms < best) {
+        best = ms;
+        best_sw = cps;
+      }
+    }
+    g.tune.sweep_ctas_per_sm = best_sw;
+  }
   g.tuned = true;
   BSP_CUDA_TRY(cudaStreamSynchronize(s));
   BSP_CUDA_TRY(cudaPeekAtLastError());
@@ -949,8 +1060,8 @@ int bsp_batch_create(bsp_handle_t h, int n_sys, const int* n_rows, const int* bs
     bsp_precond_params pp{};
     pp.kind = BSP_PC_ICHOL0;
     pp.precision = BSP_PREC_F64;
-    BSP_TRY(bsp_precond_create(h, g.A, &pp, &g.pc));
-    // tiles (never crossing a system)
+    BSP_TRY(precond_create(h, g.A, &pp, false, &g.pc));
+    // tiles (never crossing a system) and the system of each sweep task
     std::vector<int> tsys, trow, stile(g.n_sys() + 1, 0);
     for (int i = 0; i < g.n_sys(); ++i) {
       stile[i] = (int)tsys.size();
@@ -970,6 +1081,16 @@ int bsp_batch_create(bsp_handle_t h, int n_sys, const int* n_rows, const int* bs
     BSP_TRY(up(g.tile_row, trow));
     BSP_TRY(up(g.sys_tile, stile));
     BSP_TRY(up(g.sys_row, g.row_off));
+    for (int lower = 1; lower >= 0; --lower) {
+      const int nt = lower ? g.pc->n_task_lo : g.pc->n_task_up;
+      std::vector<int> rows(std::max(nt, 1)), ts(std::max(nt, 1), 0);
+      if (nt)
+        BSP_CUDA_TRY(cudaMemcpy(rows.data(), lower ? g.pc->task_lo_row.get() : g.pc->task_up_row.get(),
+                                nt * sizeof(int), cudaMemcpyDeviceToHost));
+      for (int t = 0; t < nt; ++t)
+        ts[t] = (int)(std::upper_bound(g.row_off.begin(), g.row_off.end(), (int64_t)rows[t]) - g.row_off.begin()) - 1;
+      BSP_TRY(up(lower ? g.task_sys_lo : g.task_sys_up, ts));
+    }
     BSP_TRY(g.sys_active.alloc(g.n_sys()));
     BSP_TRY(g.tickets.alloc(2));
     BSP_CUDA_TRY(cudaMemset(g.tickets.get(), 0, 2 * sizeof(unsigned)));

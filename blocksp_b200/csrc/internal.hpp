@@ -87,6 +87,7 @@ struct FactorPlan;
 // every later preconditioner built on the same matrix.
 struct SymbolicCache {
   bool valid = false;
+  bool laid_out = false;  // the sweeps' layouts were made (or found unfit)
   int64_t f_nnzb = 0;
   int n_lev_lo = 0, n_lev_up = 0, n_task_lo = 0, n_task_up = 0;
   std::vector<int64_t> h_perm;

@@ -1036,6 +1036,7 @@ static int sym_transfer(bsp_precond_s* pc, SymbolicCache& C, bool save) {
     C.n_task_lo = pc->n_task_lo;
     C.n_task_up = pc->n_task_up;
     C.valid = true;
+    C.laid_out = pc->applied;
   } else {
     pc->wv_lo = C.wv_lo;
     pc->wv_up = C.wv_up;
@@ -1349,7 +1350,7 @@ static int analyse_factor_structure(bsp_precond_s* pc, bool lower_only) {
   sweeps.lo_d = lower_only;
   sweeps.up_d = true;
   sweeps.up_trans = sweeps.up_trans_d = lower_only;
-  sweeps.start(n, pc->bs);
+  if (pc->applied) sweeps.start(n, pc->bs);
   // level orders and chain tasks on the sorted structure
   std::vector<int> order;
   auto deps_of = [](const SweepEntries& E) {
@@ -1376,7 +1377,7 @@ static int analyse_factor_structure(bsp_precond_s* pc, bool lower_only) {
 // (computed on first use), then A's values gathered into it on the device.
 static int build_factor_structure(bsp_precond_s* pc, bool lower_only) {
   SymbolicCache& C = lower_only ? pc->A->sym->ichol : pc->A->sym->ilu;
-  if (C.valid) {
+  if (C.valid && (C.laid_out || !pc->applied)) {
     BSP_TRY(sym_transfer(pc, C, false));
   } else {
     BSP_TRY(analyse_factor_structure(pc, lower_only));
@@ -2060,13 +2061,8 @@ int precond_check_status(bsp_precond_s* pc) {
   return BSP_OK;
 }
 
-}  // namespace bsp
-
-// ================================================================= C ABI
-extern "C" {
-
-int bsp_precond_create(bsp_handle_t h, bsp_matrix_t A, const bsp_precond_params* params,
-                       bsp_precond_t* out) {
+int precond_create(bsp_handle_s* h, bsp_matrix_s* A, const bsp_precond_params* params, bool applied,
+                   bsp_precond_s** out) {
   if (!h || !A || !params || !out) return BSP_INVALID;
   *out = nullptr;
   if (A->n_rows != A->n_cols) {
@@ -2094,6 +2090,7 @@ int bsp_precond_create(bsp_handle_t h, bsp_matrix_t A, const bsp_precond_params*
   pc->nu = params->sor_nu;
   pc->type = params->sor_type;
   pc->precision = params->precision;
+  pc->applied = applied;
   if (pc->kind == BSP_PC_SOR_LU || pc->kind == BSP_PC_SOR_CHOL) {
     if (pc->nu < 1) {
       record_error("SOR needs nu >= 1");
@@ -2107,6 +2104,16 @@ int bsp_precond_create(bsp_handle_t h, bsp_matrix_t A, const bsp_precond_params*
   BSP_CUDA_TRY(cudaStreamSynchronize(h->stream));
   *out = pc.release();
   return BSP_OK;
+}
+
+}  // namespace bsp
+
+// ================================================================= C ABI
+extern "C" {
+
+int bsp_precond_create(bsp_handle_t h, bsp_matrix_t A, const bsp_precond_params* params,
+                       bsp_precond_t* out) {
+  return precond_create(h, A, params, true, out);
 }
 
 int bsp_precond_destroy(bsp_precond_t pc) {

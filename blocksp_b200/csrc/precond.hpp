@@ -81,6 +81,7 @@ struct bsp_precond_s {
   std::shared_ptr<bsp::StreamSym> ss_lo, ss_up;
   bsp::StreamVals sv_lo[3], sv_up[3];
   bool level_ordered = false;  // neither's copies fitted memory
+  bool applied = true;  // false: a caller that runs the sweeps itself, no layout is made
   // elimination plan of the factorisation (shared with the matrix's cache)
   std::shared_ptr<bsp::FactorPlan> plan;
 };
@@ -88,6 +89,9 @@ struct bsp_precond_s {
 namespace bsp {
 int grid_for(const bsp_handle_s* h, int64_t n, int threads);
 int precond_build(bsp_precond_s* pc);
+// bsp_precond_create; applied: see bsp_precond_s
+int precond_create(bsp_handle_s* h, bsp_matrix_s* A, const bsp_precond_params* params, bool applied,
+                   bsp_precond_s** out);
 int precond_apply(bsp_precond_s* pc, int precision, const void* r, void* z);
 int precond_check_status(bsp_precond_s* pc);
 // out = M^-T g for an ILU0 / learned-LU preconditioner (FP64); w receives U^-T g.

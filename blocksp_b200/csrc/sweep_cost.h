@@ -85,6 +85,13 @@ inline double sweep_cost_us(SweepKernel k, int bs, int n, bool ascending, const 
   return std::sqrt(chain * chain + bulk * bulk);
 }
 
+// The batched solver's level-ordered sweep (batch_sweep.cuh) with nrhs
+// right-hand sides: a block is read once for all of them, the waits are longer.
+inline double batch_sweep_cost_us(int bs, int nrhs, int n, bool ascending, const SweepEntries& E) {
+  const double f = bs == 4 ? (nrhs == 1 ? 1.1 : 1.8) : bs == 8 ? (nrhs == 1 ? 1.2 : 1.9) : (nrhs == 1 ? 1.4 : 3.3);
+  return f * sweep_cost_us(SweepKernel::kPolled, bs, n, ascending, E);
+}
+
 // The lock-step sweep is taken when it is estimated at less than this share of
 // the other.  Over those patterns and eight block sizes it is then taken nowhere
 // where it was measured slower by more than 1.2, but for one chain of 8 x 8 rows

@@ -5,11 +5,7 @@
 
 namespace bsp {
 
-// Rows above which the two sweeps are planned on a thread each (starting one
-// takes about as long as planning 200 rows).
-constexpr int kThreadRows = 2000;
-
-template <class F> static std::future<void> run_beside(bool beside, F f) {
+std::future<void> run_beside(bool beside, std::function<void()> f) {
   if (beside) {
     try {
       return std::async(std::launch::async, f);
@@ -17,11 +13,6 @@ template <class F> static std::future<void> run_beside(bool beside, F f) {
     }
   }
   return std::async(std::launch::deferred, f);
-}
-template <class F, class G> static void both(bool beside, F f, G g) {
-  std::future<void> other = run_beside(beside, f);
-  g();
-  other.get();
 }
 
 void SweepPlanner::plan() {

@@ -1,11 +1,24 @@
 // sweep_plan.hpp — lays the two triangular sweeps of a preconditioner out.
 #pragma once
+#include <functional>
 #include <future>
 #include "sweep_cost.h"
 #include "sweep_stream.hpp"
 #include "sweep_wave.hpp"
 
 namespace bsp {
+
+// f and g, on a thread each when `beside` (a thread that cannot be had: one
+// after the other).
+std::future<void> run_beside(bool beside, std::function<void()> f);
+template <class F, class G> void both(bool beside, F f, G g) {
+  std::future<void> other = run_beside(beside, f);
+  g();
+  other.get();
+}
+// Rows above which the two sweeps are planned on a thread each (starting one
+// takes about as long as planning 200 rows).
+constexpr int kThreadRows = 2000;
 
 // The forward and the backward sweep of a factor, or of SOR on A's own blocks.
 // start() hands the host work (estimates, then the layout of the kernel that

@@ -33,7 +33,7 @@ template <int BS, int R = 1> struct WaveDim {
   static constexpr int kFetchWarps = R == 1 && BS <= 4 ? 3 : 2;
   // measured on systems of one super-task (a line, a band); several right-hand
   // sides: on batches of 2D grids
-  static constexpr double kStepUs = R > 1      ? (BS == 4 ? 0.45 : 0.65)
+  static constexpr double kStepUs = R > 1      ? (BS == 4 ? 0.45 : BS == 8 ? 0.65 : 1.2)
                                     : BS <= 2  ? 0.26
                                     : BS <= 4  ? 0.3
                                     : BS == 5  ? 0.36

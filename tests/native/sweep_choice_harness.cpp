@@ -14,14 +14,18 @@ extern "C" void sweep_shape(int bs, int nrhs, int* out) {
 
 // 1 when the lock-step sweep is taken; out: its estimate, the other kernel's,
 // super-tasks, their levels and steps planned before it was given up.  Rows of
-// different groups (n_group + 1 first rows) are independent systems.
-extern "C" int sweep_choice(int n, int ascending, int bs, int nrhs, int streamed, int limited, const int* ptr,
+// different groups (n_group + 1 first rows) are independent systems.  The other
+// kernel: 0 level-ordered, 1 streamed, 2 the batched solver's.
+extern "C" int sweep_choice(int n, int ascending, int bs, int nrhs, int other_kernel, int limited, const int* ptr,
                             const int* col, int n_group, const int* group_beg, double* out) {
   SweepEntries E;
   E.ptr.assign(ptr, ptr + n + 1);
   E.col.assign(col, col + ptr[n]);
   for (int t = 0; t < ptr[n]; ++t) E.blk.push_back(t);
-  const double other = sweep_cost_us(streamed ? SweepKernel::kStreamed : SweepKernel::kPolled, bs, n, ascending != 0, E);
+  const double other =
+      other_kernel == 2
+          ? batch_sweep_cost_us(bs, nrhs, n, ascending != 0, E)
+          : sweep_cost_us(other_kernel ? SweepKernel::kStreamed : SweepKernel::kPolled, bs, n, ascending != 0, E);
   WavePlan P;
   const std::vector<int> gb(group_beg, group_beg + (n_group ? n_group + 1 : 0));
   const double limit = kWaveShare * other;

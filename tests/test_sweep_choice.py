@@ -130,6 +130,28 @@ def test_the_faster_kernel_is_chosen(choice, name, bs, lock_step):
     assert took == [lock_step] * 2
 
 
+def together(patterns):
+    beg = np.concatenate([[0], np.cumsum([n for n, _ in patterns])])
+    return (int(beg[-1]), np.concatenate([e + b for (_, e), b in zip(patterns, beg)])), beg.astype(np.int32)
+
+
+@pytest.mark.parametrize("bs", [4, 8, 16])
+@pytest.mark.parametrize("nrhs", [1, 4])
+@pytest.mark.parametrize("name,lock_step", [("grid2d", True), ("grid3d", True), ("random2d", False), ("random3d", False),
+                                            ("graph", False)])
+def test_the_faster_kernel_is_chosen_in_a_batch(choice, name, lock_step, bs, nrhs):
+    parts = {"grid2d": [grid((100 + 3 * i, 90)) for i in range(6)], "grid3d": [grid((20, 20, 12 + i)) for i in range(6)],
+             "random2d": [randomly(grid((100 + 3 * i, 90)), i) for i in range(6)],
+             "random3d": [randomly(grid((20, 20, 12 + i)), i) for i in range(6)],
+             "graph": [graph(9000 + 100 * i, 3, i) for i in range(6)]}[name]
+    pattern, beg = together(parts)
+    for asc in (True, False):
+        n, ptr, col = csr(pattern, asc)
+        o = np.zeros(5)
+        took = choice.sweep_choice(n, int(asc), bs, nrhs, 2, 1, p(ptr), p(col), len(parts), p(beg), p(o))
+        assert bool(took) == lock_step, o
+
+
 @pytest.mark.parametrize("bs", [4, 8])
 def test_a_plan_that_is_too_slow_is_given_up_early(choice, bs):
     """The estimate grows with the super-tasks planned: a random order is left
