@@ -814,7 +814,11 @@ int build_sweeps(bsp_batch_s* B, BatchGroup& g, int R) {
 int alloc_state(bsp_batch_s* B, BatchGroup& g, int R, int hist_cap) {
   if (g.R != R) {
     const size_t nv = (size_t)g.n_rows() * R * g.bs;
-    if (!g.R || (g.R == 1) != (R == 1)) BSP_TRY(build_sweeps(B, g, R));  // the plans for 2 and 4 are the same
+    // until all of it is there the group has no state: a call that runs out of
+    // memory half way leaves nothing that a kept graph or plan could be run on
+    const int had = g.R;
+    g.R = 0;
+    if (!had || (had == 1) != (R == 1)) BSP_TRY(build_sweeps(B, g, R));  // the plans for 2 and 4 are the same
     for (DevBuf<double>* v : {&g.x, &g.r, &g.z, &g.p, &g.q}) {
       BSP_TRY(v->alloc(nv));
       BSP_CUDA_TRY(cudaMemset(v->get(), 0, nv * sizeof(double)));
@@ -837,6 +841,7 @@ int alloc_state(bsp_batch_s* B, BatchGroup& g, int R, int hist_cap) {
     g.hist_cap = -1;
   }
   if (g.hist_cap != hist_cap) {
+    g.hist_cap = -1;
     if (hist_cap > 0) BSP_TRY(g.hist.alloc((size_t)g.n_sys() * R * hist_cap));
     else g.hist.release();
     g.hist_cap = hist_cap;
