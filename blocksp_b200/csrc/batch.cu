@@ -530,9 +530,11 @@ struct bsp_batch_s {
   cudaStream_t cap = nullptr;
   cudaStream_t gs[kBatchMaxGroups] = {};
   cudaEvent_t fork = nullptr, join[kBatchMaxGroups] = {};
-  // cached graphs (valid for graph_R / graph_hist / graph_mode)
+  // cached graphs (valid for graph_R / graph_hist / graph_mode / graph_spin: the
+  // kernels' arguments are part of them)
   cudaGraphExec_t exec = nullptr, exec_body = nullptr;
   int graph_R = 0, graph_hist = -1, graph_mode = -1;
+  unsigned graph_spin = 0;
   int64_t init_kernels = 0, body_kernels = 0;
   ~bsp_batch_s() {
     if (exec) cudaGraphExecDestroy(exec);
@@ -1151,7 +1153,8 @@ int bsp_batch_pcg_dev(bsp_handle_t h, bsp_batch_t B, int nrhs, const double* b, 
   for (size_t gi = 0; gi < B->groups.size(); ++gi)
     if (!kernels_for(B->groups[gi].bs, nrhs, ks[gi])) return BSP_INVALID;
   const int hist_cap = o->hist_cap > 0 ? o->hist_cap : 0;
-  bool rebuild = B->graph_R != nrhs || B->graph_hist != hist_cap || B->graph_mode != o->mode || o->retune;
+  bool rebuild = B->graph_R != nrhs || B->graph_hist != hist_cap || B->graph_mode != o->mode ||
+                 B->graph_spin != h->spin_limit || o->retune;
   for (auto& g : B->groups) {
     if (g.R != nrhs || g.hist_cap != hist_cap) rebuild = true;
     BSP_TRY(alloc_state(B, g, nrhs, hist_cap));
@@ -1164,6 +1167,7 @@ int bsp_batch_pcg_dev(bsp_handle_t h, bsp_batch_t B, int nrhs, const double* b, 
     B->graph_R = nrhs;
     B->graph_hist = hist_cap;
     B->graph_mode = o->mode;
+    B->graph_spin = h->spin_limit;
   }
   const double setup_ms =
       rebuild ? std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_setup).count() : 0.0;
