@@ -40,8 +40,7 @@ FALLBACK_HBM_GBS = 6650.0
 TOL = 1e-10
 GOLDEN = ROOT / "tests" / "golden"
 # ncu DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of one ILU0
-# application at 64^3 with 8x8 FP64 blocks (its two sweeps), from the
-# committed capture summarised in profiles/sweep_wave_ilu0_64cube_bs8.md
+# application at 64^3 with 8x8 FP64 blocks (its two lock-step sweeps)
 ILU_APPLY_TRAFFIC_64 = 1_013_830_144  # 439.1 MB forward + 574.7 MB backward
 
 

@@ -6,7 +6,8 @@
 //   SOR                  :116-240 -> nu sync-free forward / backward sweeps from x = 0
 //   ILU0::factor         :274-291 -> k_factor mode ILU0 (row-wise, level scheduled)
 //   ILU0::invmul         :294-349 -> unit-L forward sweep + U backward sweep
-//                                    (sweep_wave.cu; here for other block sizes)
+//                                    (sweep_wave.cu, sweep_stream.cu or here, by
+//                                    the pattern: sweep_cost.h)
 //   IChol0::factor       :393-429 -> k_factor mode ICHOL0
 //   IChol0::invmul       :432-489 -> L forward sweep + L^T backward sweep
 //

@@ -5,8 +5,8 @@
 // roles:
 //   * two sets of 8 compute warps run the plan's steps in turn, in lock step,
 //     one hardware barrier a step.  A block is spread over G lanes (a 16 x 16
-//     block over two warps) that read it as 16-byte pieces straight into
-//     registers, DEPTH turns of their set ahead.  After the barrier they read
+//     block over one warp, over two with several right-hand sides) that read it
+//     as 16-byte pieces straight into registers, DEPTH turns of their set ahead.  After the barrier they read
 //     the operands of their items (rows of earlier steps, the right-hand side,
 //     external rows) from shared memory, multiply, reduce over the lanes that
 //     share a block row, and leave the row in shared memory for the next step.
@@ -30,12 +30,12 @@
 // reduction, one after another), on large systems too: at 64^3 with 8 x 8 blocks
 // DRAM is 37 to 44 % busy and the issue slots 20 %, and two stalls of three are
 // at the step barrier.  Every block is read once.  One application (two sweeps
-// and the preparation), measured against the kernels this replaced
-// (level-ordered polling rows; for 8 x 8 and 16 x 16 blocks chains that polled
-// shared memory):
+// and the preparation), measured against the kernels it takes the place of on
+// these patterns (level-ordered polling rows; for 8 x 8 and 16 x 16 blocks chains
+// that poll shared memory; sweep_cost.h has the patterns where those stay ahead):
 //   ILU0   64^3, 8 x 8           377 -> 300 us (3.2 TB/s)
 //   ILU0   48^3, 16 x 16         720 -> 351 us
-//   IChol0 300 x 257, 4 x 4     4825 -> 360 us (556 levels, twice)
+//   IChol0 300 x 257, 4 x 4     4940 -> 362 us (556 levels, twice)
 //   ILU0   40 x 36 x 44, 4 x 4   718 -> 125 us
 //   IChol0 64 x 64, 4 x 4        704 ->  85 us
 //   IChol0 24 x 20, 2 x 2        273 ->  39 us

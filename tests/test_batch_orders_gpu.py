@@ -65,3 +65,30 @@ def test_a_group_swept_by_levels_gives_up_its_waits(handle):
     again, info = B.pcg(s.b, 1, 1e-10, 500)
     assert info["status"] == 0 and np.array_equal(x, again)
     B.close()
+
+
+@pytest.mark.parametrize("batch_first", [True, False])
+def test_batch_and_preconditioner_share_a_pattern(handle, batch_first):
+    """A batch of one system has the pattern of the system's own matrix, whose
+    analysis it shares without the layout of the sweeps: whichever comes first,
+    the preconditioner applies as the oracle's and the batch solves."""
+    import blocksp_b200 as bsp
+    s = system(grid((41, 37)), 8, 11)
+    Ao = O.BSR.from_system(s)
+    want = O.IChol0(Ao)(s.b.copy())
+
+    def batch():
+        B = bsp.Batch([s], handle)
+        x, info = B.pcg(s.b, 1, 1e-10, 500)
+        assert info["status"] == 0 and rel(x, O.pcg(Ao, s.b, 1e-10, O.IChol0(Ao), 500).x) <= 1e-8
+        B.close()
+
+    def precond():
+        A = bsp.Matrix.from_system(s, handle)
+        pc = bsp.IChol0(A)
+        assert rel(pc.apply_host(s.b), want) <= 1e-11
+        pc.close()
+        A.close()
+
+    for f in ((batch, precond, precond, batch) if batch_first else (precond, batch, batch, precond)):
+        f()
